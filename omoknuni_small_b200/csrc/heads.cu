@@ -1,16 +1,11 @@
-// Policy and value heads (sm_100a, fp32 CUDA cores; < 1 % of the network's
-// arithmetic with the 2-channel / 1-channel heads).
+// Policy and value heads (sm_100a, fp32).
 //
 //   head_conv_kernel   1x1 convolution (+ folded BatchNorm, ReLU) of both heads
 //                      from the tower's board tensor; writes fp32 activations
 //                      in the reference's flatten order c * S*S + y * S + x
 //                      (src/nn/resnet_model.cpp:183,209 view({B,-1}) on NCHW).
-//   fc_kernel          out[b][j] = act(sum_i in[b][i] * WT[i][j] + bias[j]);
-//                      register-tiled (32 boards x 64 outputs per CTA, 4 x 4 per
-//                      thread, cp.async pipeline), weight matrix stored transposed.
-//   fc_pair_kernel     the policy FC and the value head's first FC as one launch.
-//   head_tails_kernel  in-place softmax over the rows of logits, and value_fc2 + tanh, as one launch.
-//   value_out_kernel   value_fc2 + tanh (one warp per board), for the value head on its own.
+//   head_fc_kernel     the policy FC and the value head's first FC (head_fc.cu), tensor cores.
+//   head_tails_kernel  their partial sums -> logits, softmax, value_fc2 + tanh, as one launch.
 #include "internal.h"
 #include "sm100_ptx.cuh"
 #include <mutex>
@@ -34,7 +29,7 @@ template <int HCT>
 __global__ void __launch_bounds__(kHeadThreads)
 head_conv_kernel(const uint8_t* __restrict__ tower, const float* __restrict__ w,
                  const float* __restrict__ bias, int HC, int pc, float* __restrict__ hp,
-                 float* __restrict__ hv, int B, int S, int C, int f16) {
+                 float* __restrict__ hv, int hp_pitch, int hv_pitch, int B, int S, int C, int f16) {
     extern __shared__ float w_s[];  // HCT == 0: [HC][C] folded weights then [HC] biases
     const int lane = threadIdx.x & 31, sub = lane >> 3, blk = lane & 7;
     if (HCT == 0) {
@@ -43,7 +38,7 @@ head_conv_kernel(const uint8_t* __restrict__ tower, const float* __restrict__ w,
         __syncthreads();
     }
     const int hc = HCT > 0 ? HCT : HC;
-    const int S2 = S * S, GP = S + 1, slots = GP * GP, vc = hc - pc;
+    const int S2 = S * S, GP = S + 1, slots = GP * GP;
     const int total = B * slots;
     const int slices = C >> 6;
     const size_t row_bytes = (size_t)C * 2;
@@ -82,8 +77,8 @@ head_conv_kernel(const uint8_t* __restrict__ tower, const float* __restrict__ w,
         }
         if (real) {
             const float o = fmaxf(keep + bh, 0.0f);
-            if (h < pc) hp[((size_t)b * pc + h) * S2 + cell] = o;
-            else hv[((size_t)b * vc + (h - pc)) * S2 + cell] = o;
+            if (h < pc) hp[(size_t)b * hp_pitch + h * S2 + cell] = o;
+            else hv[(size_t)b * hv_pitch + (h - pc) * S2 + cell] = o;
         }
     };
     if (HCT > 0) {
@@ -129,128 +124,6 @@ head_conv_kernel(const uint8_t* __restrict__ tower, const float* __restrict__ w,
     }
 }
 
-// out[b][j] = act(sum_i in[b][i] * WT[i][j] + bias[j]).  Register-tiled: a CTA owns 32 boards x
-// 64 outputs, a thread 4 boards x 4 outputs.  The 256 threads form two groups of 128 that each
-// take half of the inner dimension and run their own 3-stage cp.async pipeline of 16-deep tiles
-// (operands read back from shared memory as float4: 2 shared loads feed 16 multiply-adds); the
-// second group's sums pass through shared memory to the first, which applies bias / ReLU.
-constexpr int kFcTileB = 32, kFcTileN = 64, kFcTileK = 16, kFcStages = 3, kFcAPitch = kFcTileB + 4;
-struct FcStage {
-    float a[kFcTileK][kFcAPitch];   // inputs, k-major; the pad spreads the staging writes over banks
-    float b[kFcTileK][kFcTileN];    // weights
-};
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-struct FcProblem {
-    const float* in;     // [B][K]
-    const float* WT;     // [K][Nout]
-    const float* bias;   // [Nout]
-    float* out;          // [B][Nout]
-    int K, Nout, relu;
-};
-__device__ __forceinline__ void fc_tile(FcStage (*st)[kFcStages], const float* __restrict__ in, const float* __restrict__ WT,
-                                        const float* __restrict__ bias, float* __restrict__ out, int B, int K, int Nout,
-                                        int relu, int tile_b, int tile_n) {
-    const int half = threadIdx.x >> 7, t = threadIdx.x & 127;
-    const int b0 = tile_b * kFcTileB, n0 = tile_n * kFcTileN;
-    const int tb = (t >> 4) * 4, tn = (t & 15) * 4;   // 8 x 16 threads
-    const int tiles = (K + kFcTileK - 1) / kFcTileK, split = (tiles + 1) / 2;
-    const int first = half ? split : 0, last = half ? tiles : split;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-    auto issue = [&](int tile, int slot) {
-        if (tile < last) {
-            FcStage& s = st[half][slot];
-            const int k0 = tile * kFcTileK;
-#pragma unroll
-            for (int r = 0; r < (kFcTileK * kFcTileB) / 128; ++r) {
-                const int idx = t + r * 128;
-                const int bb = idx / kFcTileK, kk = idx - bb * kFcTileK;   // threads walk k: rows of `in`
-                const int gb = b0 + bb, gk = k0 + kk;
-                if (gb < B && gk < K) cp_async4(&s.a[kk][bb], in + (size_t)gb * K + gk);
-                else s.a[kk][bb] = 0.0f;
-            }
-#pragma unroll
-            for (int r = 0; r < (kFcTileK * kFcTileN) / 128; ++r) {
-                const int idx = t + r * 128;
-                const int kk = idx / kFcTileN, nn = idx - kk * kFcTileN;
-                const int gk = k0 + kk, gn = n0 + nn;
-                if (gk < K && gn < Nout) cp_async4(&s.b[kk][nn], WT + (size_t)gk * Nout + gn);
-                else s.b[kk][nn] = 0.0f;
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int s = 0; s < kFcStages - 1; ++s) issue(first + s, s);
-    for (int tile = first; tile < last; ++tile) {
-        const int slot = (tile - first) % kFcStages;
-        asm volatile("cp.async.wait_group %0;" ::"n"(kFcStages - 2) : "memory");
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");   // tile landed; previous slot free
-        issue(tile + kFcStages - 1, (slot + kFcStages - 1) % kFcStages);
-        const FcStage& s = st[half][slot];
-#pragma unroll
-        for (int kk = 0; kk < kFcTileK; ++kk) {
-            const float4 av = *reinterpret_cast<const float4*>(&s.a[kk][tb]);
-            const float4 bv = *reinterpret_cast<const float4*>(&s.b[kk][tn]);
-            const float aa[4] = {av.x, av.y, av.z, av.w}, bb[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    float* red = reinterpret_cast<float*>(&st[0][0]);   // 128 x 16 floats, reusing the stages
-    if (half) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) red[(i * 4 + j) * 128 + t] = acc[i][j];
-    }
-    __syncthreads();
-    if (half) return;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gb = b0 + tb + i;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tn + j;
-            if (gb >= B || gn >= Nout) continue;
-            float v = acc[i][j] + red[(i * 4 + j) * 128 + t] + bias[gn];
-            if (relu) v = fmaxf(v, 0.0f);
-            out[(size_t)gb * Nout + gn] = v;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256)
-fc_kernel(const float* __restrict__ in, const float* __restrict__ WT, const float* __restrict__ bias,
-          float* __restrict__ out, int B, int K, int Nout, int relu) {
-    __shared__ __align__(16) FcStage st[2][kFcStages];
-    fc_tile(st, in, WT, bias, out, B, K, Nout, relu, blockIdx.x, blockIdx.y);
-}
-
-// Two independent layers over the same boards in one launch (the policy FC and the value head's first FC): the
-// first tiles_n0 values of blockIdx.y are output tiles of problem 0, the rest of problem 1.  Each output is
-// computed exactly as fc_kernel computes it.
-__global__ void __launch_bounds__(256)
-fc_pair_kernel(FcProblem p0, FcProblem p1, int B, int tiles_n0) {
-    __shared__ __align__(16) FcStage st[2][kFcStages];
-    asm volatile("griddepcontrol.wait;" ::: "memory");               // the inputs come from the kernel ahead in the stream
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const bool first = (int)blockIdx.y < tiles_n0;
-    const FcProblem& p = first ? p0 : p1;
-    fc_tile(st, p.in, p.WT, p.bias, p.out, B, p.K, p.Nout, p.relu, blockIdx.x, first ? blockIdx.y : blockIdx.y - tiles_n0);
-}
-
 __device__ __forceinline__ float block_reduce(float v, bool is_max, float* red) {
     for (int off = 16; off > 0; off >>= 1) {
         const float o = __shfl_xor_sync(0xffffffffu, v, off);
@@ -265,112 +138,132 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float* red) 
     return v;
 }
 
-__global__ void __launch_bounds__(256)
-value_out_kernel(const float* __restrict__ hidden, const float* __restrict__ w2, float b2, int H, int B,
-                 float* __restrict__ value) {
-    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (b >= B) return;
-    float s = 0.0f;
-    for (int i = lane; i < H; i += 32) s = fmaf(hidden[(size_t)b * H + i], w2[i], s);
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) value[b] = tanhf(s + b2);
+// Element j of row b of a layer's result: its slices of partial sums added in the layer's fixed order, fifteen loads
+// (five groups of three, or fifteen groups) in flight at a time.
+constexpr int kSliceBatch = 15;
+static_assert(kSliceBatch % kHeadFcGroup == 0, "a batch of slices is a whole number of groups");
+template <int GROUP>
+__device__ __forceinline__ float sum_slices_in(const HeadFcLayer& l, const float* p, size_t step) {
+    float total = 0.0f;
+    for (int s = 0; s < l.slices; s += kSliceBatch) {
+        float v[kSliceBatch];
+#pragma unroll
+        for (int k = 0; k < kSliceBatch; ++k) v[k] = s + k < l.slices ? __ldcg(p + (size_t)(s + k) * step) : 0.0f;
+#pragma unroll
+        for (int g = 0; g < kSliceBatch; g += GROUP) {
+            if (s + g >= l.slices) break;
+            float group = v[g];
+#pragma unroll
+            for (int k = g + 1; k < g + GROUP; ++k)
+                if (s + k < l.slices) group = __fadd_rn(group, v[k]);
+            total = s + g ? __fadd_rn(total, group) : group;
+        }
+    }
+    return total;
+}
+__device__ __forceinline__ float sum_slices(const HeadFcLayer& l, int b, int B, int j) {
+    const float* p = l.part + (size_t)b * l.part_pitch + j;
+    const size_t step = (size_t)B * l.part_pitch;
+    if (l.slices == 1) return __ldcg(p);
+    return l.slice_group == 1 ? sum_slices_in<1>(l, p, step) : sum_slices_in<kHeadFcGroup>(l, p, step);
 }
 
-// The tails of both heads in one launch, started as a programmatic dependent of fc_pair_kernel: CTAs
-// [0, softmax_rows) normalise one row of logits each (maximum, sum of exponentials, division), the rest finish four boards' values
-// each as value_out_kernel does (a warp per board).
-__global__ void __launch_bounds__(128)
-head_tails_kernel(float* __restrict__ logits, int A, int softmax_rows, const float* __restrict__ hidden,
-                  const float* __restrict__ w2, float b2, int H, int B, float* __restrict__ value) {
-    __shared__ float red[4];
+// The tails of both heads in one launch, started as a programmatic dependent of the FC kernel: CTAs [0, policy_rows)
+// finish one row of logits each (sum of the slices, bias, softmax: maximum, sum of exponentials, division), the rest
+// one board's value each.  A thread per output: what a small batch waits for is the trip to L2 for the slices.
+constexpr int kTailThreads = 256;
+constexpr int kTailRegs = 2;             // logits a thread keeps in registers: rows of up to 512
+__global__ void __launch_bounds__(kTailThreads)
+head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __restrict__ logits, int A, int policy_rows, int softmax,
+                  const HeadFcLayer val, const float* __restrict__ b1, const float* __restrict__ w2, float b2, int H, int B,
+                  float* __restrict__ value) {
+    __shared__ float red[kTailThreads / 32];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if ((int)blockIdx.x < softmax_rows) {
-        float* row = logits + (size_t)blockIdx.x * A;
+    if ((int)blockIdx.x < policy_rows) {
+        const int b = blockIdx.x;
+        float* row = logits + (size_t)b * A;
+        if (A <= kTailRegs * kTailThreads) {
+            float x[kTailRegs];
+            float m = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < kTailRegs; ++k) {
+                const int i = threadIdx.x + k * kTailThreads;
+                x[k] = -INFINITY;
+                if (i < A) x[k] = pol.part ? __fadd_rn(sum_slices(pol, b, B, i), bp[i]) : row[i];
+                m = fmaxf(m, x[k]);
+            }
+            float scale = 1.0f;
+            if (softmax) {
+                m = block_reduce(m, true, red);
+                float s = 0.0f;
+#pragma unroll
+                for (int k = 0; k < kTailRegs; ++k)
+                    if ((int)threadIdx.x + k * kTailThreads < A) { x[k] = expf(x[k] - m); s += x[k]; }
+                scale = 1.0f / block_reduce(s, false, red);
+            }
+#pragma unroll
+            for (int k = 0; k < kTailRegs; ++k) {
+                const int i = threadIdx.x + k * kTailThreads;
+                if (i < A) row[i] = x[k] * scale;
+            }
+            return;
+        }
         float m = -INFINITY;
-        for (int i = threadIdx.x; i < A; i += blockDim.x) m = fmaxf(m, row[i]);
+        for (int i = threadIdx.x; i < A; i += kTailThreads) {
+            if (pol.part) row[i] = __fadd_rn(sum_slices(pol, b, B, i), bp[i]);
+            m = fmaxf(m, row[i]);
+        }
+        if (!softmax) return;
         m = block_reduce(m, true, red);
         float s = 0.0f;
-        for (int i = threadIdx.x; i < A; i += blockDim.x) s += expf(row[i] - m);
+        for (int i = threadIdx.x; i < A; i += kTailThreads) s += expf(row[i] - m);
         s = block_reduce(s, false, red);
         const float inv = 1.0f / s;
-        for (int i = threadIdx.x; i < A; i += blockDim.x) row[i] = expf(row[i] - m) * inv;
+        for (int i = threadIdx.x; i < A; i += kTailThreads) row[i] = expf(row[i] - m) * inv;
     } else {
-        const int b = ((int)blockIdx.x - softmax_rows) * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-        if (b >= B) return;
+        const int b = (int)blockIdx.x - policy_rows;
         float s = 0.0f;
-        for (int i = lane; i < H; i += 32) s = fmaf(hidden[(size_t)b * H + i], w2[i], s);
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (lane == 0) value[b] = tanhf(s + b2);
+        for (int i = threadIdx.x; i < H; i += kTailThreads) s = fmaf(fmaxf(__fadd_rn(sum_slices(val, b, B, i), b1[i]), 0.0f), w2[i], s);
+        s = block_reduce(s, false, red);
+        if (threadIdx.x == 0) value[b] = tanhf(s + b2);
     }
 }
 
 }  // namespace
 
-// The FC part of both heads in two launches: {policy FC (when policy_in is given), value FC1 + ReLU}, then
-// {softmax over the logits (when asked), value FC2 + tanh}.  The FC results equal launch_fc / launch_value_out on
-// the same buffers bit for bit.
-int launch_head_fcs(const float* policy_in, const float* WpT, const float* bp, float* policy_out, int policy_k, int policy_size,
-                    int softmax, const float* value_in, const float* W1T, const float* b1, float* hidden, int value_k, int H,
-                    const float* w2, float b2, float* value_out, int B, cudaStream_t st) {
-    const FcProblem p0{policy_in, WpT, bp, policy_out, policy_k, policy_size, 0};
-    const FcProblem p1{value_in, W1T, b1, hidden, value_k, H, 1};
-    const int tiles0 = policy_in ? (policy_size + kFcTileN - 1) / kFcTileN : 0, tiles1 = (H + kFcTileN - 1) / kFcTileN;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((B + kFcTileB - 1) / kFcTileB, tiles0 + tiles1);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    OB200_CUDA_OK(cudaLaunchKernelEx(&cfg, fc_pair_kernel, p0, p1, B, tiles0));
-    counters().launches.fetch_add(1, std::memory_order_relaxed);
-    const int rows = softmax ? B : 0;
-    cfg.gridDim = dim3((unsigned)(rows + (B + 3) / 4));
-    cfg.blockDim = dim3(128);
-    OB200_CUDA_OK(cudaLaunchKernelEx(&cfg, head_tails_kernel, policy_out, policy_size, rows, (const float*)hidden, w2, b2, H, B, value_out));
+int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_out, int policy_size, int softmax,
+                      const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
+                      cudaStream_t st) {
+    const int rows = policy_out && (policy.part || softmax) ? B : 0;
+    OB200_CUDA_OK(launch_dependent(head_tails_kernel, dim3((unsigned)(rows + B)), dim3(kTailThreads), 0, st, policy, bp,
+                                   policy_out, policy_size, rows, softmax, value, b1, w2, b2, H, B, value_out));
     counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
 }
 
 int launch_head_conv(const void* tower, const float* w, const float* bias, int HC, int pc,
-                     float* hp, float* hv, int B, int S, cudaStream_t st, int C, int dtype) {
+                     float* hp, float* hv, int hp_pitch, int hv_pitch, int B, int S, cudaStream_t st, int C, int dtype) {
     const int f16 = dtype == OB200_DTYPE_F16;
     if (C < 64 || C % 64) return set_error(OB200_ERR_INVALID, "head conv: tower channels %d not a multiple of 64", C);
     const long long total = (long long)B * (S + 1) * (S + 1);   // positions, one warp per 32
     const unsigned grid = (unsigned)((total + kHeadThreads - 1) / kHeadThreads);
     const uint8_t* t = static_cast<const uint8_t*>(tower);
     switch (HC) {
-        case 1: head_conv_kernel<1><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, B, S, C, f16); break;
-        case 2: head_conv_kernel<2><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, B, S, C, f16); break;
-        case 3: head_conv_kernel<3><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, B, S, C, f16); break;
-        case 4: head_conv_kernel<4><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, B, S, C, f16); break;
+        case 1: head_conv_kernel<1><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
+        case 2: head_conv_kernel<2><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
+        case 3: head_conv_kernel<3><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
+        case 4: head_conv_kernel<4><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
         default: {
             const size_t smem = (size_t)(HC * C + HC) * sizeof(float);
             if (smem > 200 * 1024)
                 return set_error(OB200_ERR_UNSUPPORTED, "head conv: %d head channels x %d tower channels exceed shared memory", HC, C);
             if (smem > 48 * 1024)
                 OB200_CUDA_OK(cudaFuncSetAttribute(head_conv_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            head_conv_kernel<0><<<grid, kHeadThreads, smem, st>>>(t, w, bias, HC, pc, hp, hv, B, S, C, f16);
+            head_conv_kernel<0><<<grid, kHeadThreads, smem, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16);
         }
     }
     OB200_LAUNCHED("head_conv_kernel");
-    return OB200_OK;
-}
-
-int launch_fc(const float* in, const float* WT, const float* bias, float* out, int B, int K, int Nout, int relu,
-              cudaStream_t st) {
-    dim3 grid((B + kFcTileB - 1) / kFcTileB, (Nout + kFcTileN - 1) / kFcTileN);
-    fc_kernel<<<grid, 256, 0, st>>>(in, WT, bias, out, B, K, Nout, relu);
-    OB200_LAUNCHED("fc_kernel");
-    return OB200_OK;
-}
-
-int launch_value_out(const float* hidden, const float* w2, float b2, int H, int B, float* value, cudaStream_t st) {
-    value_out_kernel<<<(B * 32 + 255) / 256, 256, 0, st>>>(hidden, w2, b2, H, B, value);
-    OB200_LAUNCHED("value_out_kernel");
     return OB200_OK;
 }
 
@@ -403,7 +296,7 @@ static int value_head_scratch_ptr(float** out) {
     return OB200_OK;
 }
 
-int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const float* W1T,
+int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const HeadFcLayer& value_layer,
                              const float* b1, const float* w2, float b2, int H, int B, int S, float* value_out,
                              cudaStream_t st, int dtype) {
     const size_t need = (size_t)B * ((size_t)vc * S * S + (size_t)H);
@@ -416,9 +309,13 @@ int launch_value_head_static(const void* tower, const float* vw, const float* vb
     float* hv = scratch;                                  // [B][vc * S * S]
     float* hidden = scratch + (size_t)B * vc * S * S;     // [B][H]
     // every element read below is written first by the launch before it: nothing needs clearing
-    if (int rc = launch_head_conv(tower, vw, vb, vc, 0, hv, hv, B, S, st, 64, dtype)) return rc;
-    if (int rc = launch_fc(hv, W1T, b1, hidden, B, vc * S * S, H, 1, st)) return rc;
-    return launch_value_out(hidden, w2, b2, H, B, value_out, st);
+    if (int rc = launch_head_conv(tower, vw, vb, vc, 0, hv, hv, 0, vc * S * S, B, S, st, 64, dtype)) return rc;
+    // the layer with all its chunks in one CTA per tile: one slice, which fits the scratch
+    HeadFcLayer l = value_layer;
+    l.in = hv; l.in_pitch = vc * S * S; l.part = hidden; l.part_pitch = H;
+    l.chunks_per_slice = l.chunks; l.slices = 1; l.slice_group = 1;
+    if (int rc = launch_head_fc(&l, 1, B, st)) return rc;
+    return launch_head_tails(HeadFcLayer{}, nullptr, nullptr, 0, 0, l, b1, H, w2, b2, value_out, B, st);
 }
 
 }  // namespace ob200

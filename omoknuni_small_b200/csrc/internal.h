@@ -45,7 +45,7 @@ int tower_resident_head_channels_max();
 int launch_conv_tower_resident(const BoardTensorMap& in_map, const BoardTensorMap& out_map, const void* layers_dev,
                                int n_layers, int B, int S, cudaStream_t st, const float* head_w = nullptr,
                                const float* head_b = nullptr, int head_ch = 0, int head_pc = 0, float* hp = nullptr,
-                               float* hv = nullptr, int dtype = 0, const int16_t* enc_hist = nullptr,
+                               float* hv = nullptr, int hp_pitch = 0, int hv_pitch = 0, int dtype = 0, const int16_t* enc_hist = nullptr,
                                const uint8_t* enc_nh = nullptr, const uint8_t* enc_tm = nullptr, int enc_planes = 0);
 // Towers of 128 / 256 channels (tower_wide.cu): cin a multiple of 64 up to 256, cout 128 or 256,
 // taps 9 (3x3) or 1 (1x1).  in_map: boxes of conv_wide_box_rows() rows over a cin-channel tensor;
@@ -60,17 +60,33 @@ int launch_conv_wide_maps(const BoardTensorMap& in_map, const BoardTensorMap& ou
                           cudaStream_t st, float* out_f32 = nullptr, int dtype = 0);
 
 // C: channels of the tower board tensor (a multiple of 64); w: [HC][C]
+// hp [B][hp_pitch], hv [B][hv_pitch]: a board's policy / value head channels, flattened as c * S*S + y * S + x
 int launch_head_conv(const void* tower, const float* w, const float* bias, int HC, int pc, float* hp,
-                     float* hv, int B, int S, cudaStream_t st, int C = 64, int dtype = 0);
-int launch_fc(const float* in, const float* WT, const float* bias, float* out, int B, int K, int Nout, int relu,
-              cudaStream_t st);
-// Both heads' FC layers in two launches ({policy FC, value FC1}, {softmax, value FC2 + tanh}); policy_in may be
-// null (a policy that is already in policy_out); results as the single-layer launchers give them.
-int launch_head_fcs(const float* policy_in, const float* WpT, const float* bp, float* policy_out, int policy_k, int policy_size,
-                    int softmax, const float* value_in, const float* W1T, const float* b1, float* hidden, int value_k, int H,
-                    const float* w2, float b2, float* value_out, int B, cudaStream_t st);
-int launch_value_out(const float* hidden, const float* w2, float b2, int H, int B, float* value, cudaStream_t st);
-int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const float* W1T,
+                     float* hv, int hp_pitch, int hv_pitch, int B, int S, cudaStream_t st, int C = 64, int dtype = 0);
+// A fully connected layer of a head on the tensor cores in fp32 precision (head_fc.cu): its sums leave as `slices`
+// partial results [slice][B][part_pitch], to be added in order - in runs of slice_group first, when that is above 1.
+constexpr int kHeadFcGroup = 3;
+struct HeadFcLayer {
+    const float* in;          // [B][in_pitch]
+    int in_pitch, K;
+    const uint8_t* w;         // head_fc_pack
+    int n_tiles, k_blocks, chunk_k, chunks, chunks_per_slice, slices, slice_group;
+    float* part;
+    int part_pitch;           // outputs beyond it are dropped
+    int part_vec;             // set by the launcher: rows may be written 16 bytes at a time
+};
+size_t head_fc_packed_bytes(int K, int N);
+int head_fc_pack(const float* w_dev, int K, int N, void* packed_dev, cudaStream_t st);   // w [N][K] on the device
+void head_fc_shape(HeadFcLayer* l, int K, int N);
+int head_fc_plan(HeadFcLayer* l, int n_layers, int B, int sms);
+int launch_head_fc(const HeadFcLayer* layers, int n_layers, int B, cudaStream_t st);
+// What is left of both heads in one launch: partial sums + bias -> logits (or softmax of them), partial sums + bias ->
+// ReLU -> value FC2 -> tanh.  policy.part may be null: the logits are in policy_out already (convolution planes).
+int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_out, int policy_size, int softmax,
+                      const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
+                      cudaStream_t st);
+// value_layer: the value head's first FC (its in / part fields are filled in here)
+int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const HeadFcLayer& value_layer,
                              const float* b1, const float* w2, float b2, int H, int B, int S, float* value_out,
                              cudaStream_t st, int dtype = 0);
 size_t value_head_static_capacity();

@@ -42,9 +42,10 @@ struct ob200_net {
     int sm_count = 148;
     // device: heads
     float *head_w = nullptr, *head_b = nullptr;      // [pc+vc][64], [pc+vc]
-    float *WpT = nullptr, *bp = nullptr, *W1T = nullptr, *b1 = nullptr, *w2 = nullptr;
+    float *bp = nullptr, *b1 = nullptr, *w2 = nullptr;
     float b2 = 0.0f;
-    float *hp = nullptr, *hv = nullptr, *hidden = nullptr;
+    float *hp = nullptr, *hv = nullptr;               // head channels, rows of a multiple of four floats (fc_*.in_pitch)
+    ob200::HeadFcLayer fc_policy{}, fc_value{};             // policy FC, value FC1
     // device: policy as convolution planes (policy_kind 1): 1x1 convolution on the tensor cores
     void* pol_w = nullptr; float* pol_b = nullptr; float* pol_planes = nullptr; int pol_cout = 0;
     // device + pinned host staging of the host-buffer calls.  Two calls may be in flight per handle: while the
@@ -143,6 +144,32 @@ int add_conv(ob200_net* n, const std::string& conv, const std::string& bn, int c
     if (int rc = upload(n, &db, shift)) return rc;
     n->conv_w.push_back(dw); n->conv_b.push_back(db);
     return OB200_OK;
+}
+
+int add_head_fc(ob200_net* n, HeadFcLayer* l, const std::vector<float>& w, int K, int N) {
+    // the fp32 matrix is needed on the device only until it is split
+    float* plain = nullptr;
+    uint8_t* dw = nullptr;
+    if (int rc = dev_alloc(n, &dw, head_fc_packed_bytes(K, N), false)) return rc;
+    OB200_CUDA_OK(cudaMalloc(&plain, w.size() * sizeof(float)));
+    cudaError_t e = cudaMemcpy(plain, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice);
+    const int rc = e == cudaSuccess ? head_fc_pack(plain, K, N, dw, nullptr) : OB200_OK;
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    cudaFree(plain);
+    OB200_CUDA_OK(e);
+    if (rc) return rc;
+    head_fc_shape(l, K, N);
+    l->w = dw;
+    l->in_pitch = (K + 3) / 4 * 4;
+    l->part_pitch = (N + 3) / 4 * 4;
+    return OB200_OK;
+}
+
+// The FC layers a forward runs, in launch order: {policy FC, value FC1}, or the latter alone.
+int head_fc_layers(const ob200_net* n, HeadFcLayer (&l)[2]) {
+    if (n->cfg.policy_kind == OB200_POLICY_CONV_PLANES) { l[0] = n->fc_value; return 1; }
+    l[0] = n->fc_policy; l[1] = n->fc_value;
+    return 2;
 }
 
 // One tower layer on the kernel that covers the handle's width.
@@ -255,6 +282,7 @@ int ob200_net_finalize(ob200_net* n) {
     if (n->finalized) return set_error(OB200_ERR_STATE, "ob200_net_finalize: already finalised");
     const ob200_net_config& c = n->cfg;
     OB200_CUDA_OK(cudaSetDevice(c.device));
+    OB200_CUDA_OK(cudaDeviceGetAttribute(&n->sm_count, cudaDevAttrMultiProcessorCount, c.device));
     const int F = c.filters, S2 = c.board_size * c.board_size, pc = c.policy_head_ch, vc = c.value_head_ch;
     // tower
     if (int rc = add_conv(n, "input_conv", "input_bn", c.input_channels, n->cin_pad)) return rc;
@@ -279,7 +307,7 @@ int ob200_net_finalize(ob200_net* n) {
     for (int h = 0; h < vc; ++h) { for (int k = 0; k < F; ++k) hw[(size_t)(pch + h) * F + k] = (*vw)[(size_t)h * F + k] * vs[h]; hb[pch + h] = vb[h]; }
     if (int rc = upload(n, &n->head_w, hw)) return rc;
     if (int rc = upload(n, &n->head_b, hb)) return rc;
-    // fully connected layers, stored transposed ([in][out]) for coalesced reads
+    // fully connected layers
     const int Kp = pc * S2, Kv = vc * S2, A = c.policy_size, H = c.value_hidden;
     if (planes_policy) {
         // policy planes: 1x1 convolution with bias, no BatchNorm, no ReLU, run on the tensor cores with the
@@ -301,18 +329,14 @@ int ob200_net_finalize(ob200_net* n) {
     } else {
         if (int rc = need(n, "policy_fc.weight", (size_t)A * Kp, &fcw)) return rc;
         if (int rc = need(n, "policy_fc.bias", (size_t)A, &fcb)) return rc;
-        std::vector<float> wpt((size_t)Kp * A);
-        for (int j = 0; j < A; ++j) for (int i = 0; i < Kp; ++i) wpt[(size_t)i * A + j] = (*fcw)[(size_t)j * Kp + i];
-        if (int rc = upload(n, &n->WpT, wpt)) return rc;
+        if (int rc = add_head_fc(n, &n->fc_policy, *fcw, Kp, A)) return rc;
         if (int rc = upload(n, &n->bp, *fcb)) return rc;
     }
     if (int rc = need(n, "value_fc1.weight", (size_t)H * Kv, &f1w)) return rc;
     if (int rc = need(n, "value_fc1.bias", (size_t)H, &f1b)) return rc;
     if (int rc = need(n, "value_fc2.weight", (size_t)H, &f2w)) return rc;
     if (int rc = need(n, "value_fc2.bias", 1, &f2b)) return rc;
-    std::vector<float> w1t((size_t)Kv * H);
-    for (int j = 0; j < H; ++j) for (int i = 0; i < Kv; ++i) w1t[(size_t)i * H + j] = (*f1w)[(size_t)j * Kv + i];
-    if (int rc = upload(n, &n->W1T, w1t)) return rc;
+    if (int rc = add_head_fc(n, &n->fc_value, *f1w, Kv, H)) return rc;
     if (int rc = upload(n, &n->b1, *f1b)) return rc;
     if (int rc = upload(n, &n->w2, *f2w)) return rc;
     n->b2 = (*f2b)[0];
@@ -352,9 +376,6 @@ int ob200_net_finalize(ob200_net* n) {
         if (int rc = dev_alloc(n, &n->fused_done, (size_t)L, true)) return rc;
         n->fused = !(env && env[0] == '0');
         n->fused_forced = env && env[0] == '2';
-        int dev = 0;
-        OB200_CUDA_OK(cudaGetDevice(&dev));
-        OB200_CUDA_OK(cudaDeviceGetAttribute(&n->sm_count, cudaDevAttrMultiProcessorCount, dev));
     }
     if (!n->wide && n->cin_pad == 64 && tower_resident_smem_bytes(c.board_size, 1 + 2 * c.blocks) != 0) {
         // boards stay in shared memory through all the layers: one ordinary launch, whole-board boxes
@@ -374,9 +395,25 @@ int ob200_net_finalize(ob200_net* n) {
         n->resident = env ? env[0] != '0' : std::getenv("OB200_TOWER_FUSED") == nullptr;
     }
     const size_t MB = c.max_batch;
-    if (int rc = dev_alloc(n, &n->hp, MB * (planes_policy ? 1 : Kp), false)) return rc;
-    if (int rc = dev_alloc(n, &n->hv, MB * Kv, false)) return rc;
-    if (int rc = dev_alloc(n, &n->hidden, MB * H, false)) return rc;
+    if (!planes_policy) {
+        if (int rc = dev_alloc(n, &n->hp, MB * n->fc_policy.in_pitch, true)) return rc;
+        n->fc_policy.in = n->hp;
+    }
+    if (int rc = dev_alloc(n, &n->hv, MB * n->fc_value.in_pitch, true)) return rc;
+    n->fc_value.in = n->hv;
+    // partial sums of the FC layers: room for the batch size that needs the most of them
+    size_t pol_part = 0, val_part = 0;
+    for (int m = 1; m <= (c.max_batch + 127) / 128; ++m) {
+        const int B = std::min(c.max_batch, m * 128);
+        HeadFcLayer l[2];
+        const int nl = head_fc_layers(n, l);
+        head_fc_plan(l, nl, B, n->sm_count);
+        val_part = std::max(val_part, (size_t)l[nl - 1].slices * B * l[nl - 1].part_pitch);
+        if (nl == 2) pol_part = std::max(pol_part, (size_t)l[0].slices * B * l[0].part_pitch);
+    }
+    if (int rc = dev_alloc(n, &n->fc_value.part, val_part, false)) return rc;
+    if (pol_part)
+        if (int rc = dev_alloc(n, &n->fc_policy.part, pol_part, false)) return rc;
     for (auto& sl : n->slot) {
         if (int rc = dev_alloc(n, &sl.d_policy, MB * A, false)) return rc;
         if (int rc = dev_alloc(n, &sl.d_value, MB, false)) return rc;
@@ -436,7 +473,7 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
         const bool with_heads = heads_done && c.policy_kind != OB200_POLICY_CONV_PLANES && hc <= tower_resident_head_channels_max();
         const int rc = launch_conv_tower_resident(own_input ? n->in_map_board : board_map, n->out_map_board, n->resident_layers,
                                                   1 + 2 * c.blocks, B, S, st, n->head_w, n->head_b, with_heads ? hc : 0,
-                                                  with_heads ? c.policy_head_ch : 0, n->hp, n->hv, c.tower_dtype,
+                                                  with_heads ? c.policy_head_ch : 0, n->hp, n->hv, n->fc_policy.in_pitch, n->fc_value.in_pitch, c.tower_dtype,
                                                   gomoku ? gomoku->hist : nullptr, gomoku ? gomoku->nh : nullptr,
                                                   gomoku ? gomoku->tm : nullptr, c.input_channels);
         if (rc == OB200_OK) { done = true; x = 0; n->tower_path = 2; if (heads_done) *heads_done = with_heads; }
@@ -501,15 +538,17 @@ int forward_device(ob200_net* n, const void* input_bt, int B, float* policy_out,
         policy_planes_gather_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
             n->pol_planes, n->pol_cout, pc, B, S, policy_out);
         OB200_LAUNCHED("policy_planes_gather_kernel");
-        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, vc, 0, n->hv, n->hv, B, S, st, F, c.tower_dtype)) return rc;
+        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, vc, 0, n->hv, n->hv, 0, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
     } else if (!heads_done) {
-        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, pc + vc, pc, n->hp, n->hv, B, S, st, F, c.tower_dtype)) return rc;
+        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, pc + vc, pc, n->hp, n->hv, n->fc_policy.in_pitch, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
     }
     // the FC layers of both heads: {policy FC, value FC1} in one launch, {softmax, value FC2 + tanh} in the next
-    const bool fc_policy = c.policy_kind != OB200_POLICY_CONV_PLANES;
-    if (int rc = launch_head_fcs(fc_policy ? n->hp : nullptr, n->WpT, n->bp, policy_out, pc * S2, c.policy_size,
-                                 out_kind == OB200_OUT_PROBS, n->hv, n->W1T, n->b1, n->hidden, vc * S2, c.value_hidden, n->w2,
-                                 n->b2, value_out, B, st)) return rc;
+    HeadFcLayer l[2];
+    const int nl = head_fc_layers(n, l);
+    head_fc_plan(l, nl, B, n->sm_count);
+    if (int rc = launch_head_fc(l, nl, B, st)) return rc;
+    if (int rc = launch_head_tails(nl == 2 ? l[0] : HeadFcLayer{}, n->bp, policy_out, c.policy_size, out_kind == OB200_OUT_PROBS,
+                                   l[nl - 1], n->b1, c.value_hidden, n->w2, n->b2, value_out, B, st)) return rc;
     counters().evals.fetch_add((uint64_t)B, std::memory_order_relaxed);
     counters().batches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
@@ -749,7 +788,7 @@ int ob200_net_value_head_noalloc(ob200_net* n, const void* tower_board_tensor, i
     if (c.filters != 64)
         return set_error(OB200_ERR_UNSUPPORTED, "ob200_net_value_head_noalloc: covers towers of 64 filters");
     return launch_value_head_static(tower_board_tensor, n->head_w + (size_t)pc * c.filters, n->head_b + pc,
-                                    c.value_head_ch, n->W1T, n->b1, n->w2, n->b2, c.value_hidden, B, c.board_size,
+                                    c.value_head_ch, n->fc_value, n->b1, n->w2, n->b2, c.value_hidden, B, c.board_size,
                                     value_out, as_stream(stream), c.tower_dtype);
 }
 

@@ -80,8 +80,8 @@ struct ResidentParams {
     const float* head_w;      // [head_ch][64]
     const float* head_b;      // [head_ch]
     int head_ch, head_pc;     // channels in all, and how many of them belong to the policy head
-    float* hp;                // [B][head_pc][S*S]
-    float* hv;                // [B][head_ch - head_pc][S*S]
+    float *hp, *hv;           // [B][pitch]: channel c of a cell at c * S*S + cell
+    int hp_pitch, hv_pitch;
     // optional: the tower's input comes from Gomoku move histories instead of an input tensor - the epilogue
     // threads write each board's input rows themselves (the planes of ob200_launch_encode_gomoku).  enc_hist == null: off.
     const int16_t* enc_hist;  // [B][16] k-th most recent move
@@ -151,7 +151,7 @@ __device__ __forceinline__ void write_input_row(uint8_t* dst_row, int row, bool 
 // over eight consecutive channels each, added as ((0+1)+(2+3))+((4+5)+(6+7)), then the bias, then ReLU.
 template <bool F16>
 __device__ __noinline__ void head_row(const uint8_t* row_ptr, int row, const float* head_s, int head_ch, int head_pc,
-                                      int board, int S, int GP, float* hp, float* hv) {
+                                      int board, int S, int GP, float* hp, float* hv, int hp_pitch, int hv_pitch) {
     float a[kC];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -175,8 +175,8 @@ __device__ __noinline__ void head_row(const uint8_t* row_ptr, int row, const flo
         }
         const float sum = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
         const float o = fmaxf(sum + head_s[kHeadMax * kC + h], 0.0f);
-        if (h < head_pc) hp[((size_t)board * head_pc + h) * S2 + cell] = o;
-        else hv[((size_t)board * (head_ch - head_pc) + (h - head_pc)) * S2 + cell] = o;
+        if (h < head_pc) hp[(size_t)board * hp_pitch + h * S2 + cell] = o;
+        else hv[(size_t)board * hv_pitch + (h - head_pc) * S2 + cell] = o;
     }
 }
 __device__ __forceinline__ void store_zero_row(uint8_t* dst_row) {
@@ -398,7 +398,7 @@ conv_tower_resident_kernel(const __grid_constant__ CUtensorMap in_map, const __g
                     else if (has_res) store_half_row<true, F16, 4>(dst_row, row, r, bias_t, res);
                     else store_half_row<false, F16, 4>(dst_row, row, r, bias_t, res);
                     if (l + 1 == L && p.head_ch > 0 && valid)
-                        head_row<F16>(dst_row, row, head_s, p.head_ch, p.head_pc, board_of(round, bd), p.S, p.GP, p.hp, p.hv);
+                        head_row<F16>(dst_row, row, head_s, p.head_ch, p.head_pc, board_of(round, bd), p.S, p.GP, p.hp, p.hv, p.hp_pitch, p.hv_pitch);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // rows -> the tensor cores' / the store's reads
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
@@ -471,7 +471,7 @@ int tower_resident_head_channels_max() { return kHeadMax; }
 // tower's output ride along in the last epilogue; results as launch_head_conv writes them.
 int launch_conv_tower_resident(const BoardTensorMap& in_map, const BoardTensorMap& out_map, const void* layers_dev,
                                int n_layers, int B, int S, cudaStream_t st, const float* head_w, const float* head_b,
-                               int head_ch, int head_pc, float* hp, float* hv, int dtype, const int16_t* enc_hist,
+                               int head_ch, int head_pc, float* hp, float* hv, int hp_pitch, int hv_pitch, int dtype, const int16_t* enc_hist,
                                const uint8_t* enc_nh, const uint8_t* enc_tm, int enc_planes) {
     if (enc_hist && (!enc_nh || !enc_tm || (enc_planes != 17 && enc_planes != 19) || ((uintptr_t)enc_hist & 15)))
         return set_error(OB200_ERR_INVALID, "resident tower: bad move-history arguments (17 or 19 planes, histories 16-byte aligned)");
@@ -503,7 +503,7 @@ int launch_conv_tower_resident(const BoardTensorMap& in_map, const BoardTensorMa
     p.layers = static_cast<const ResidentLayer*>(layers_dev); p.n_layers = n_layers; p.B = B; p.S = S; p.GP = S + 1; p.slots = slots;
     p.error = device_error_word();
     if (!p.error) return set_error(OB200_ERR_CUDA, "resident tower: cannot resolve the device error word");
-    p.head_w = head_w; p.head_b = head_b; p.head_ch = head_ch; p.head_pc = head_pc; p.hp = hp; p.hv = hv;
+    p.head_w = head_w; p.head_b = head_b; p.head_ch = head_ch; p.head_pc = head_pc; p.hp = hp; p.hv = hv; p.hp_pitch = hp_pitch; p.hv_pitch = hv_pitch;
     p.enc_hist = enc_hist; p.enc_nh = enc_nh; p.enc_tm = enc_tm; p.enc_planes = enc_planes;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(B < sms ? B : sms); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
