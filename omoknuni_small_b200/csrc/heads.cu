@@ -8,120 +8,121 @@
 //   head_tails_kernel  their partial sums -> logits, softmax, value_fc2 + tanh, as one launch.
 #include "internal.h"
 #include "sm100_ptx.cuh"
+#include "head_conv.cuh"
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 namespace ob200 {
 namespace {
 
-struct alignas(16) Pack8 { uint32_t v[4]; };
+using namespace ptx;
 
-// A warp takes 32 consecutive positions of the board tensor (pad positions included, their
-// results are dropped).  Eight lanes share a position: lane = 8 * (position within a group of 4)
-// + channel block, so a warp-wide 16-byte load covers 4 positions x 128 contiguous bytes of one
-// 64-channel slice and the 8 loads of a warp are issued back to back.  Each lane multiplies its
-// 8 channels (per slice) into a head channel's partial sum, three shuffle steps add the 8 lanes,
-// and lane (sub, blk) keeps the sum of group blk: after 8 groups every lane owns one position and
-// stores once per head channel.  C = tower channels (a multiple of 64).
-// HCT > 0: that many head channels, partial sums of all of them held in registers while the
-// slices stream by; HCT == 0: any number, weights in shared memory, one head channel at a time.
-constexpr int kHeadThreads = 128;
-template <int HCT>
-__global__ void __launch_bounds__(kHeadThreads)
-head_conv_kernel(const uint8_t* __restrict__ tower, const float* __restrict__ w,
-                 const float* __restrict__ bias, int HC, int pc, float* __restrict__ hp,
-                 float* __restrict__ hv, int hp_pitch, int hv_pitch, int B, int S, int C, int f16) {
-    extern __shared__ float w_s[];  // HCT == 0: [HC][C] folded weights then [HC] biases
-    const int lane = threadIdx.x & 31, sub = lane >> 3, blk = lane & 7;
-    if (HCT == 0) {
-        for (int i = threadIdx.x; i < HC * C; i += blockDim.x) w_s[i] = w[i];
-        for (int i = threadIdx.x; i < HC; i += blockDim.x) w_s[HC * C + i] = bias[i];
+// A CTA takes tiles of 128 consecutive positions of the board tensor (pad positions included, their results are
+// dropped): rows of 128 bytes per 64-channel slice into swizzled shared memory, two MMAs per 16 channels and slice
+// (see head_conv.cuh; the same products in the same order as the board-resident tower's last layer), accumulators to
+// the flattened head activations.  blockIdx.y: the group of up to 64 head channels.  HBM-bound for large batches (it
+// reads the tower's output once per group); several CTAs an SM cover one another's latency.
+constexpr int kConvThreads = 256;
+constexpr int kConvTile = 128;
+constexpr int kConvTmemCols = 128;
+struct HeadConvParams {
+    const uint8_t* tower;
+    HeadConvWeights head;
+    float *hp, *hv;
+    int hp_pitch, hv_pitch;
+    int B, S, slices, tiles;
+    int* error;
+};
+template <bool F16>
+__global__ void __launch_bounds__(kConvThreads)
+head_conv_kernel(const HeadConvParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t bars[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_s;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h0 = (int)blockIdx.y * 64, hc = min(64, p.head.hc - h0), rows = (hc + 15) / 16 * 16;
+    uint8_t* a_s = smem;                                                // [slice][128 rows][128 bytes]
+    uint8_t* w_s = smem + p.slices * kConvTile * 128;                   // [slice][split term][rows][128 bytes]
+    const uint32_t w_bytes = (uint32_t)(p.slices * 3 * rows * 128);
+    const uint32_t w_full = smem_u32(&bars[0]), done = smem_u32(&bars[1]);
+    volatile int* abort_flag = &abort_s;
+    if (threadIdx.x == 0) {
+        mbar_init(w_full, 1); mbar_init(done, 1);
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_arrive_expect_tx(w_full, w_bytes);
+        bulk_g2s(smem_u32(w_s), p.head.w + (size_t)blockIdx.y * p.slices * 3 * 64 * 128, w_bytes, w_full);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)kConvTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_slot;
+    OB200_PDL_ENTER();
+    const int GP = p.S + 1, slots = GP * GP, S2 = p.S * p.S, total = p.B * slots;
+    const size_t row_bytes = (size_t)p.slices * 128;
+    const uint32_t id2 = make_idesc(F16, kConvTile, 2 * rows), id1 = make_idesc(F16, kConvTile, rows);
+    const int q = warp & 3, half = warp >> 2;
+    uint32_t phase = 0;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, phase ^= 1u) {
+        // the tensor is padded to whole tiles: every row is readable
+        const uint8_t* src = p.tower + ((size_t)OB200_GUARD + (size_t)tile * kConvTile) * row_bytes;
+        for (int i = threadIdx.x; i < p.slices * kConvTile * 8; i += kConvThreads) {
+            const int c = i & 7, sl = (i >> 3) % p.slices, r = (i >> 3) / p.slices;
+            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)r * row_bytes + sl * 128 + c * 16));
+            *reinterpret_cast<uint4*>(a_s + (sl * kConvTile + r) * 128 + ((c ^ (r & 7)) << 4)) = v;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");    // the previous tile's accumulators have been read
         __syncthreads();
-    }
-    const int hc = HCT > 0 ? HCT : HC;
-    const int S2 = S * S, GP = S + 1, slots = GP * GP;
-    const int total = B * slots;
-    const int slices = C >> 6;
-    const size_t row_bytes = (size_t)C * 2;
-    const int p0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-    if (p0 >= total) return;
-    // the tensor's trailing guard positions make the (at most 31) positions past the end readable
-    const uint8_t* src = tower + ((size_t)OB200_GUARD + p0 + sub) * row_bytes + blk * 16;
-    float a[8][8];
-    auto load_slice = [&](int sl) {
+        if (threadIdx.x == 0) {
+            if (mbar_wait(w_full, 0, abort_flag)) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a = desc_lo(smem_u32(a_s)), w = desc_lo(smem_u32(w_s));
+                for (int sl = 0; sl < p.slices; ++sl)
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const Pack8 v = *reinterpret_cast<const Pack8*>(src + (size_t)it * 4 * row_bytes + (size_t)sl * 128);
+                    for (int ks = 0; ks < 4; ++ks) {
+                        const uint32_t at = a + (uint32_t)(sl * kConvTile * 8 + ks * 2), wt = w + (uint32_t)(sl * 3 * rows * 8 + ks * 2);
+                        umma(tmem_base, at, wt, id2, (sl | ks) ? 1u : 0u);
+                        umma(tmem_base + (uint32_t)rows, at, wt + (uint32_t)(2 * rows * 8), id1, 1u);
+                    }
+                umma_commit(done);
+            } else { abort_s = 1; atomicExch(p.error, 4); }
+        }
+        bool good = mbar_wait(done, phase, abort_flag);
+        if (!__syncthreads_and(good)) { if (threadIdx.x == 0) atomicExch(p.error, 3); break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int pos = tile * kConvTile + q * 32 + lane;
+        const int b = pos / slots, r = pos - b * slots, y = r / GP, x = r - y * GP;
+        const bool real = pos < total && y < p.S && x < p.S;
+        const int cell = y * p.S + x;
+        const uint32_t t = tmem_base + ((uint32_t)(q * 32) << 16);
+        for (int c = half; c < rows / 8; c += 2) {
+            uint32_t big[8], small[8];
+            tmem_ld8(t + c * 8, big);
+            tmem_ld8(t + rows + c * 8, small);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // the tower's storage type: both conversions are exact
-                if (f16) ptx::unpack2<true>(v.v[j], a[it][2 * j], a[it][2 * j + 1]);
-                else ptx::unpack2<false>(v.v[j], a[it][2 * j], a[it][2 * j + 1]);
+            for (int j = 0; j < 8; ++j) {
+                const int h = h0 + c * 8 + j;
+                if (c * 8 + j >= hc || !real) continue;
+                const float o = head_conv_value(__uint_as_float(big[j]), __uint_as_float(small[j]), __ldg(p.head.scale + h), __ldg(p.head.bias + h));
+                if (h < p.head.pc) p.hp[(size_t)b * p.hp_pitch + h * S2 + cell] = o;
+                else p.hv[(size_t)b * p.hv_pitch + (h - p.head.pc) * S2 + cell] = o;
             }
-        }
-    };
-    // this lane's own position: group blk, member sub
-    const int p = p0 + blk * 4 + sub;
-    const int b = p / slots, r = p - b * slots;
-    const int y = r / GP, x = r - y * GP;
-    const bool real = p < total && y < S && x < S;
-    const int cell = y * S + x;
-    auto finish = [&](int h, const float (&part)[8], float bh) {
-        float keep = 0.0f;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            float s = part[it];
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            keep = (it == blk) ? s : keep;
-        }
-        if (real) {
-            const float o = fmaxf(keep + bh, 0.0f);
-            if (h < pc) hp[(size_t)b * hp_pitch + h * S2 + cell] = o;
-            else hv[(size_t)b * hv_pitch + (h - pc) * S2 + cell] = o;
-        }
-    };
-    if (HCT > 0) {
-        constexpr int kRegCh = HCT > 0 ? HCT : 1;
-        float part[kRegCh][8];
-#pragma unroll
-        for (int h = 0; h < kRegCh; ++h)
-#pragma unroll
-            for (int it = 0; it < 8; ++it) part[h][it] = 0.0f;
-        for (int sl = 0; sl < slices; ++sl) {
-            load_slice(sl);
-#pragma unroll
-            for (int h = 0; h < kRegCh; ++h) {
-                const float4* wr = reinterpret_cast<const float4*>(w + (size_t)h * C + sl * 64 + blk * 8);
-                const float4 w0 = __ldg(wr), w1 = __ldg(wr + 1);
-                const float wk[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-                for (int it = 0; it < 8; ++it)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) part[h][it] = fmaf(a[it][k], wk[k], part[h][it]);
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < kRegCh; ++h) finish(h, part[h], __ldg(bias + h));
-    } else {
-        if (slices == 1) load_slice(0);
-        for (int h = 0; h < hc; ++h) {
-            float part[8];
-#pragma unroll
-            for (int it = 0; it < 8; ++it) part[it] = 0.0f;
-            for (int sl = 0; sl < slices; ++sl) {
-                if (slices > 1) load_slice(sl);   // re-read per head channel (L1 / L2 hits)
-                const float4* wr = reinterpret_cast<const float4*>(w_s + (size_t)h * C + sl * 64 + blk * 8);
-                const float4 w0 = wr[0], w1 = wr[1];
-                const float wk[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-                for (int it = 0; it < 8; ++it)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) part[it] = fmaf(a[it][k], wk[k], part[it]);
-            }
-            finish(h, part, w_s[hc * C + h]);
         }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kConvTmemCols) : "memory");
 }
 
 __device__ __forceinline__ float block_reduce(float v, bool is_max, float* red) {
@@ -242,28 +243,74 @@ int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_
     return OB200_OK;
 }
 
-int launch_head_conv(const void* tower, const float* w, const float* bias, int HC, int pc,
-                     float* hp, float* hv, int hp_pitch, int hv_pitch, int B, int S, cudaStream_t st, int C, int dtype) {
-    const int f16 = dtype == OB200_DTYPE_F16;
-    if (C < 64 || C % 64) return set_error(OB200_ERR_INVALID, "head conv: tower channels %d not a multiple of 64", C);
-    const long long total = (long long)B * (S + 1) * (S + 1);   // positions, one warp per 32
-    const unsigned grid = (unsigned)((total + kHeadThreads - 1) / kHeadThreads);
-    const uint8_t* t = static_cast<const uint8_t*>(tower);
-    switch (HC) {
-        case 1: head_conv_kernel<1><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
-        case 2: head_conv_kernel<2><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
-        case 3: head_conv_kernel<3><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
-        case 4: head_conv_kernel<4><<<grid, kHeadThreads, 0, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16); break;
-        default: {
-            const size_t smem = (size_t)(HC * C + HC) * sizeof(float);
-            if (smem > 200 * 1024)
-                return set_error(OB200_ERR_UNSUPPORTED, "head conv: %d head channels x %d tower channels exceed shared memory", HC, C);
-            if (smem > 48 * 1024)
-                OB200_CUDA_OK(cudaFuncSetAttribute(head_conv_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            head_conv_kernel<0><<<grid, kHeadThreads, smem, st>>>(t, w, bias, HC, pc, hp, hv, hp_pitch, hv_pitch, B, S, C, f16);
+size_t head_conv_packed_bytes(int hc, int C) {
+    const int last = hc % 64, rows = hc / 64 * 64 + (last + 15) / 16 * 16;
+    return (size_t)rows * 3 * C * 2;
+}
+
+void head_conv_pack(const float* w, int hc, int C, int dtype, void* packed_out, float* scale_out) {
+    std::memset(packed_out, 0, head_conv_packed_bytes(hc, C));
+    const int slices = C / 64;
+    for (int h = 0; h < hc; ++h) {
+        const int group = h / 64, row = h % 64, in_group = hc - group * 64 < 64 ? hc - group * 64 : 64, rows = (in_group + 15) / 16 * 16;
+        // fp16: bring the channel's largest weight to [2^12, 2^13), a power of two that the result is divided by
+        float up = 1.0f;
+        if (dtype == OB200_DTYPE_F16) {
+            float top = 0.0f;
+            for (int k = 0; k < C; ++k) top = std::max(top, std::fabs(w[(size_t)h * C + k]));
+            int e = 0;
+            if (top > 0.0f && std::isfinite(top)) { std::frexp(top, &e); up = std::ldexp(1.0f, std::min(13 - e, 100)); }
+        }
+        scale_out[h] = 1.0f / up;
+        for (int k = 0; k < C; ++k) {
+            float v = w[(size_t)h * C + k] * up;
+            uint8_t* at = static_cast<uint8_t*>(packed_out) + ((size_t)group * slices * 64 + (size_t)(k / 64) * rows) * 3 * 128 + row * 128 +
+                          ((((k & 63) >> 3) ^ (row & 7)) << 4) + (k & 7) * 2;
+            for (int t = 0; t < 3; ++t) {
+                uint16_t u;
+                float f;
+                if (dtype == OB200_DTYPE_F16) {
+                    u = f32_to_f16_rne_sat(v);
+                    f = __half2float(*reinterpret_cast<const __half*>(&u));
+                } else {
+                    u = f32_to_bf16_rne(v);
+                    const uint32_t b = (uint32_t)u << 16;
+                    std::memcpy(&f, &b, 4);
+                }
+                std::memcpy(at + (size_t)t * rows * 128, &u, 2);
+                v -= f;
+            }
         }
     }
-    OB200_LAUNCHED("head_conv_kernel");
+}
+
+int launch_head_conv(const void* tower, const HeadConvWeights& head, float* hp, float* hv, int hp_pitch, int hv_pitch, int B, int S,
+                     cudaStream_t st, int C, int dtype) {
+    if (C < 64 || C % 64 || C > 256 || head.hc < 1)
+        return set_error(OB200_ERR_INVALID, "head conv: tower channels %d not a multiple of 64 up to 256, or no head channels", C);
+    if (int rc = require_device()) return rc;
+    int dev = 0, sms = 0;
+    OB200_CUDA_OK(cudaGetDevice(&dev));
+    OB200_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const BoardGeom g = board_geom(S, B);
+    if (g.P > 0x7fffffffLL - kConvTile) return set_error(OB200_ERR_TOO_LARGE, "head conv: batch too large");
+    HeadConvParams p;
+    p.tower = static_cast<const uint8_t*>(tower); p.head = head; p.hp = hp; p.hv = hv; p.hp_pitch = hp_pitch; p.hv_pitch = hv_pitch;
+    p.B = B; p.S = S; p.slices = C / 64; p.tiles = (int)(g.Ppad / kConvTile);
+    p.error = device_error_word();
+    if (!p.error) return set_error(OB200_ERR_CUDA, "head conv: cannot resolve the device error word");
+    const int groups = (head.hc + 63) / 64, rows = (std::min(head.hc, 64) + 15) / 16 * 16;
+    const size_t smem = (size_t)p.slices * (kConvTile + 3 * rows) * 128 + 1024;
+    auto kernel = dtype == OB200_DTYPE_F16 ? head_conv_kernel<true> : head_conv_kernel<false>;
+    static bool configured[64][2] = {{false, false}};
+    if (dev < 0 || dev >= 64 || !configured[dev][dtype]) {
+        OB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (kConvTile + 3 * 64) * 128 + 1024));
+        if (dev >= 0 && dev < 64) configured[dev][dtype] = true;
+    }
+    // four CTAs an SM (128 TMEM columns each), where the shared memory of so many fits
+    const int per_sm = std::max(1, std::min(4, (int)(220 * 1024 / (smem + 1024))));
+    OB200_CUDA_OK(launch_dependent(kernel, dim3(std::min(p.tiles, sms * per_sm), groups), dim3(kConvThreads), smem, st, p));
+    counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
 }
 
@@ -296,9 +343,10 @@ static int value_head_scratch_ptr(float** out) {
     return OB200_OK;
 }
 
-int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const HeadFcLayer& value_layer,
+int launch_value_head_static(const void* tower, const HeadConvWeights& value_conv, const HeadFcLayer& value_layer,
                              const float* b1, const float* w2, float b2, int H, int B, int S, float* value_out,
                              cudaStream_t st, int dtype) {
+    const int vc = value_conv.hc;
     const size_t need = (size_t)B * ((size_t)vc * S * S + (size_t)H);
     if (need > kStaticScratchFloats)
         return set_error(OB200_ERR_TOO_LARGE,
@@ -309,7 +357,7 @@ int launch_value_head_static(const void* tower, const float* vw, const float* vb
     float* hv = scratch;                                  // [B][vc * S * S]
     float* hidden = scratch + (size_t)B * vc * S * S;     // [B][H]
     // every element read below is written first by the launch before it: nothing needs clearing
-    if (int rc = launch_head_conv(tower, vw, vb, vc, 0, hv, hv, 0, vc * S * S, B, S, st, 64, dtype)) return rc;
+    if (int rc = launch_head_conv(tower, value_conv, nullptr, hv, 0, vc * S * S, B, S, st, 64, dtype)) return rc;
     // the layer with all its chunks in one CTA per tile: one slice, which fits the scratch
     HeadFcLayer l = value_layer;
     l.in = hv; l.in_pitch = vc * S * S; l.part = hidden; l.part_pitch = H;

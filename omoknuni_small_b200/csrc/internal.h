@@ -33,19 +33,24 @@ size_t tower_fused_smem_bytes(int S, int n_layers);   // 0: does not fit
 int launch_conv_tower(const BoardTensorMap& stem_in_map, const void* layers_dev, int n_layers, int* flags, int tiles_pitch,
                       int* done, int epoch, int B, int S, cudaStream_t st, int dtype = 0);
 // The 64-filter tower with the boards resident in shared memory (tower_resident.cu): boards up to
-// 15x15, one ordinary launch.  in_map / out_map: boxes of tower_resident_box_rows(S) rows.
-size_t tower_resident_layer_bytes();
-void tower_resident_fill_layer(void* dst, const void* w, const float* bias, int has_res);
-int tower_resident_box_rows(int S);
-size_t tower_resident_smem_bytes(int S, int n_layers);   // 0: does not fit
+// 15x15, one ordinary launch.
+// The even and the odd columns of a 64-channel board tensor of B boards as 4-D maps (channel, pair of cells, row, board);
+// a box is one board's plane, (S + 2) / 2 pairs x (S + 1) rows, what lies outside the grid reads as zero.
+struct BoardPlaneMaps { BoardTensorMap even, odd; };
+int make_board_plane_maps(const void* base, int S, int B, BoardPlaneMaps* out);
+// The heads' 1x1 convolutions (head_conv.cuh).  w: blocks [group of up to 64 channels][64-channel K slice][split term]
+// of (channels of the group rounded up to 16) rows x 128 bytes, 128-byte swizzle; scale, bias: [hc].
+struct HeadConvWeights { const uint8_t* w; const float *scale, *bias; int hc, pc; };
+size_t head_conv_packed_bytes(int hc, int C);
+void head_conv_pack(const float* w, int hc, int C, int dtype, void* packed_out, float* scale_out);   // w [hc][C], host
+bool tower_resident_covers(int S, int n_layers);
 int tower_resident_head_channels_max();
-// head_ch > 0: the heads' 1x1 convolutions ride along in the last epilogue (results as launch_head_conv's).
-// enc_hist != null: the input is not read through in_map but written by the kernel from Gomoku move histories
+// head (optional): the heads' 1x1 convolutions come along as one more layer (results as launch_head_conv's).
+// enc_hist != null: the input is not read through `in` but written by the kernel from Gomoku move histories
 // ([B][16] int16, 16-byte aligned; history lengths and sides to move [B]; 17 or 19 planes), as launch_encode_gomoku would.
-int launch_conv_tower_resident(const BoardTensorMap& in_map, const BoardTensorMap& out_map, const void* layers_dev,
-                               int n_layers, int B, int S, cudaStream_t st, const float* head_w = nullptr,
-                               const float* head_b = nullptr, int head_ch = 0, int head_pc = 0, float* hp = nullptr,
-                               float* hv = nullptr, int hp_pitch = 0, int hv_pitch = 0, int dtype = 0, const int16_t* enc_hist = nullptr,
+int launch_conv_tower_resident(const BoardPlaneMaps& in, const BoardPlaneMaps& out, const void* const* layers_dev, const float* bias,
+                               int n_layers, int B, int S, cudaStream_t st, const HeadConvWeights* head = nullptr, float* hp = nullptr, float* hv = nullptr,
+                               int hp_pitch = 0, int hv_pitch = 0, int dtype = 0, const int16_t* enc_hist = nullptr,
                                const uint8_t* enc_nh = nullptr, const uint8_t* enc_tm = nullptr, int enc_planes = 0);
 // Towers of 128 / 256 channels (tower_wide.cu): cin a multiple of 64 up to 256, cout 128 or 256,
 // taps 9 (3x3) or 1 (1x1).  in_map: boxes of conv_wide_box_rows() rows over a cin-channel tensor;
@@ -59,10 +64,10 @@ int launch_conv_wide_maps(const BoardTensorMap& in_map, const BoardTensorMap& ou
                           const void* packed_w, const float* bias, int B, int S, int cin, int cout, int taps, int relu,
                           cudaStream_t st, float* out_f32 = nullptr, int dtype = 0);
 
-// C: channels of the tower board tensor (a multiple of 64); w: [HC][C]
+// C: channels of the tower board tensor (a multiple of 64).
 // hp [B][hp_pitch], hv [B][hv_pitch]: a board's policy / value head channels, flattened as c * S*S + y * S + x
-int launch_head_conv(const void* tower, const float* w, const float* bias, int HC, int pc, float* hp,
-                     float* hv, int hp_pitch, int hv_pitch, int B, int S, cudaStream_t st, int C = 64, int dtype = 0);
+int launch_head_conv(const void* tower, const HeadConvWeights& head, float* hp, float* hv, int hp_pitch, int hv_pitch, int B, int S,
+                     cudaStream_t st, int C = 64, int dtype = 0);
 // A fully connected layer of a head on the tensor cores in fp32 precision (head_fc.cu): its sums leave as `slices`
 // partial results [slice][B][part_pitch], to be added in order - in runs of slice_group first, when that is above 1.
 constexpr int kHeadFcGroup = 3;
@@ -86,7 +91,7 @@ int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_
                       const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
                       cudaStream_t st);
 // value_layer: the value head's first FC (its in / part fields are filled in here)
-int launch_value_head_static(const void* tower, const float* vw, const float* vb, int vc, const HeadFcLayer& value_layer,
+int launch_value_head_static(const void* tower, const HeadConvWeights& value_conv, const HeadFcLayer& value_layer,
                              const float* b1, const float* w2, float b2, int H, int B, int S, float* value_out,
                              cudaStream_t st, int dtype = 0);
 size_t value_head_static_capacity();

@@ -37,11 +37,12 @@ struct ob200_net {
     void* fused_layers = nullptr; int *fused_flags = nullptr, *fused_done = nullptr; int fused_pitch = 0, fused_epoch = 0, fused_final = 0;
     bool fused = false, fused_forced = false;   // forced: OB200_TOWER_FUSED=2 (tests: every batch size)
     // the board-resident tower (64 filters, boards up to 15x15): layer descriptors, whole-board boxes
-    void* resident_layers = nullptr; bool resident = false;
-    ob200::BoardTensorMap in_map_board{}, out_map_board{};
+    void** resident_layers = nullptr; bool resident = false;
+    std::vector<float> resident_bias;                // [1 + 2 * blocks][64]
+    ob200::BoardPlaneMaps in_planes{}, out_planes{};
     int sm_count = 148;
     // device: heads
-    float *head_w = nullptr, *head_b = nullptr;      // [pc+vc][64], [pc+vc]
+    ob200::HeadConvWeights head_conv{}, value_conv{};   // policy and value channels (FC policy head), value channels alone
     float *bp = nullptr, *b1 = nullptr, *w2 = nullptr;
     float b2 = 0.0f;
     float *hp = nullptr, *hv = nullptr;               // head channels, rows of a multiple of four floats (fc_*.in_pitch)
@@ -143,6 +144,21 @@ int add_conv(ob200_net* n, const std::string& conv, const std::string& bn, int c
     if (int rc = upload(n, &dw, packed)) return rc;
     if (int rc = upload(n, &db, shift)) return rc;
     n->conv_w.push_back(dw); n->conv_b.push_back(db);
+    return OB200_OK;
+}
+
+// w [hc][filters], b [hc]: folded 1x1 convolutions of the heads, the first pc of them the policy's.
+int add_head_conv(ob200_net* n, HeadConvWeights* out, const float* w, const float* b, int hc, int pc) {
+    const int F = n->cfg.filters;
+    std::vector<uint8_t> packed(head_conv_packed_bytes(hc, F));
+    std::vector<float> scale(hc), bias(b, b + hc);
+    head_conv_pack(w, hc, F, n->cfg.tower_dtype, packed.data(), scale.data());
+    uint8_t* dw = nullptr;
+    float *ds = nullptr, *db = nullptr;
+    if (int rc = upload(n, &dw, packed)) return rc;
+    if (int rc = upload(n, &ds, scale)) return rc;
+    if (int rc = upload(n, &db, bias)) return rc;
+    *out = HeadConvWeights{dw, ds, db, hc, pc};
     return OB200_OK;
 }
 
@@ -305,8 +321,10 @@ int ob200_net_finalize(ob200_net* n) {
     std::vector<float> hw((size_t)(pch + vc) * F), hb(pch + vc);
     for (int h = 0; h < pch; ++h) { for (int k = 0; k < F; ++k) hw[(size_t)h * F + k] = (*pw)[(size_t)h * F + k] * ps[h]; hb[h] = pb[h]; }
     for (int h = 0; h < vc; ++h) { for (int k = 0; k < F; ++k) hw[(size_t)(pch + h) * F + k] = (*vw)[(size_t)h * F + k] * vs[h]; hb[pch + h] = vb[h]; }
-    if (int rc = upload(n, &n->head_w, hw)) return rc;
-    if (int rc = upload(n, &n->head_b, hb)) return rc;
+    if (int rc = add_head_conv(n, &n->value_conv, hw.data() + (size_t)pch * F, hb.data() + pch, vc, 0)) return rc;
+    n->head_conv = n->value_conv;
+    if (!planes_policy)
+        if (int rc = add_head_conv(n, &n->head_conv, hw.data(), hb.data(), pch + vc, pch)) return rc;
     // fully connected layers
     const int Kp = pc * S2, Kv = vc * S2, A = c.policy_size, H = c.value_hidden;
     if (planes_policy) {
@@ -377,19 +395,16 @@ int ob200_net_finalize(ob200_net* n) {
         n->fused = !(env && env[0] == '0');
         n->fused_forced = env && env[0] == '2';
     }
-    if (!n->wide && n->cin_pad == 64 && tower_resident_smem_bytes(c.board_size, 1 + 2 * c.blocks) != 0) {
-        // boards stay in shared memory through all the layers: one ordinary launch, whole-board boxes
+    if (!n->wide && n->cin_pad == 64 && tower_resident_covers(c.board_size, 1 + 2 * c.blocks)) {
+        // boards stay in shared memory through all the layers: one ordinary launch
         const char* env = std::getenv("OB200_TOWER_RESIDENT");
         const int L = 1 + 2 * c.blocks;
-        std::vector<unsigned char> host(tower_resident_layer_bytes() * L);
+        if (int rc = upload(n, &n->resident_layers, n->conv_w)) return rc;
+        n->resident_bias.resize((size_t)L * F);
         for (int l = 0; l < L; ++l)
-            tower_resident_fill_layer(host.data() + tower_resident_layer_bytes() * l, n->conv_w[l], n->conv_b[l], l >= 2 && !(l & 1));
-        unsigned char* dl = nullptr;
-        if (int rc = upload(n, &dl, host)) return rc;
-        n->resident_layers = dl;
-        const int box = tower_resident_box_rows(c.board_size);
-        if (int rc = make_board_tensor_map(n->act_in, n->rows, box, &n->in_map_board, n->cin_pad)) return rc;
-        if (int rc = make_board_tensor_map(n->act[0], n->rows, box, &n->out_map_board, F)) return rc;
+            OB200_CUDA_OK(cudaMemcpy(n->resident_bias.data() + (size_t)l * F, n->conv_b[l], F * sizeof(float), cudaMemcpyDeviceToHost));
+        if (int rc = make_board_plane_maps(n->act_in, c.board_size, c.max_batch, &n->in_planes)) return rc;
+        if (int rc = make_board_plane_maps(n->act[0], c.board_size, c.max_batch, &n->out_planes)) return rc;
         // on unless switched off; an explicit choice about the single-launch tower (OB200_TOWER_FUSED, used by
         // tests and comparisons to pick one of the other two paths) also switches it off unless it is asked for
         n->resident = env ? env[0] != '0' : std::getenv("OB200_TOWER_FUSED") == nullptr;
@@ -465,15 +480,15 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
     bool done = false;
     const bool own_input = input_bt == n->act_in;
     if (n->resident) {
-        BoardTensorMap board_map;
+        BoardPlaneMaps planes;
         if (!own_input)
-            if (int rc = input_map(n, input_bt, B, tower_resident_box_rows(S), &board_map)) return rc;
-        // the heads' 1x1 convolutions ride along when they are few (FC policy head: policy + value channels)
+            if (int rc = make_board_plane_maps(input_bt, S, B, &planes)) return rc;
+        // the heads' 1x1 convolutions come along as one more layer (FC policy head: policy + value channels)
         const int hc = c.policy_head_ch + c.value_head_ch;
         const bool with_heads = heads_done && c.policy_kind != OB200_POLICY_CONV_PLANES && hc <= tower_resident_head_channels_max();
-        const int rc = launch_conv_tower_resident(own_input ? n->in_map_board : board_map, n->out_map_board, n->resident_layers,
-                                                  1 + 2 * c.blocks, B, S, st, n->head_w, n->head_b, with_heads ? hc : 0,
-                                                  with_heads ? c.policy_head_ch : 0, n->hp, n->hv, n->fc_policy.in_pitch, n->fc_value.in_pitch, c.tower_dtype,
+        const int rc = launch_conv_tower_resident(own_input ? n->in_planes : planes, n->out_planes, n->resident_layers,
+                                                  n->resident_bias.data(), 1 + 2 * c.blocks, B, S, st, with_heads ? &n->head_conv : nullptr, n->hp, n->hv,
+                                                  n->fc_policy.in_pitch, n->fc_value.in_pitch, c.tower_dtype,
                                                   gomoku ? gomoku->hist : nullptr, gomoku ? gomoku->nh : nullptr,
                                                   gomoku ? gomoku->tm : nullptr, c.input_channels);
         if (rc == OB200_OK) { done = true; x = 0; n->tower_path = 2; if (heads_done) *heads_done = with_heads; }
@@ -530,7 +545,7 @@ int forward_device(ob200_net* n, const void* input_bt, int B, float* policy_out,
     int x = 0;
     bool heads_done = false;
     if (int rc = tower_device(n, input_bt, B, &x, st, &heads_done, gomoku)) return rc;
-    const int S2 = S * S, pc = c.policy_head_ch, vc = c.value_head_ch;
+    const int S2 = S * S, pc = c.policy_head_ch;
     if (c.policy_kind == OB200_POLICY_CONV_PLANES) {
         if (int rc = launch_conv_wide_maps(n->act_load[x], n->act_load[x], nullptr, n->pol_w, n->pol_b, B, S, F, n->pol_cout, 1, 0,
                                            st, n->pol_planes, c.tower_dtype)) return rc;
@@ -538,9 +553,9 @@ int forward_device(ob200_net* n, const void* input_bt, int B, float* policy_out,
         policy_planes_gather_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
             n->pol_planes, n->pol_cout, pc, B, S, policy_out);
         OB200_LAUNCHED("policy_planes_gather_kernel");
-        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, vc, 0, n->hv, n->hv, 0, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
+        if (int rc = launch_head_conv(n->act[x], n->value_conv, nullptr, n->hv, 0, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
     } else if (!heads_done) {
-        if (int rc = launch_head_conv(n->act[x], n->head_w, n->head_b, pc + vc, pc, n->hp, n->hv, n->fc_policy.in_pitch, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
+        if (int rc = launch_head_conv(n->act[x], n->head_conv, n->hp, n->hv, n->fc_policy.in_pitch, n->fc_value.in_pitch, B, S, st, F, c.tower_dtype)) return rc;
     }
     // the FC layers of both heads: {policy FC, value FC1} in one launch, {softmax, value FC2 + tanh} in the next
     HeadFcLayer l[2];
@@ -784,11 +799,9 @@ int ob200_net_value_head_noalloc(ob200_net* n, const void* tower_board_tensor, i
     const ob200_net_config& c = n->cfg;
     OB200_CUDA_OK(cudaSetDevice(c.device));
     if (int rc = require_device()) return rc;
-    const int pc = c.policy_kind == OB200_POLICY_CONV_PLANES ? 0 : c.policy_head_ch;
     if (c.filters != 64)
         return set_error(OB200_ERR_UNSUPPORTED, "ob200_net_value_head_noalloc: covers towers of 64 filters");
-    return launch_value_head_static(tower_board_tensor, n->head_w + (size_t)pc * c.filters, n->head_b + pc,
-                                    c.value_head_ch, n->fc_value, n->b1, n->w2, n->b2, c.value_hidden, B, c.board_size,
+    return launch_value_head_static(tower_board_tensor, n->value_conv, n->fc_value, n->b1, n->w2, n->b2, c.value_hidden, B, c.board_size,
                                     value_out, as_stream(stream), c.tower_dtype);
 }
 

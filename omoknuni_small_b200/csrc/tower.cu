@@ -302,20 +302,24 @@ int* device_error_word() {
     return cached[dev];
 }
 
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeFn tensor_map_encoder() {
+    static const EncodeFn encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess ? reinterpret_cast<EncodeFn>(fn)
+                                                                                                            : nullptr;
+    }();
+    return encode;
+}
+
 // 2-D tensor map over a board tensor: inner dimension the `channels` channels of a position,
 // outer dimension `rows` positions; boxes of 64 channels (128 bytes) x box_rows, 128-byte swizzle.
 int make_board_tensor_map(const void* base, long long rows, int box_rows, BoardTensorMap* out, int channels) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
-            return set_error(OB200_ERR_CUDA, "cannot resolve cuTensorMapEncodeTiled from the driver");
-        encode = reinterpret_cast<EncodeFn>(fn);
-    }
+    const EncodeFn encode = tensor_map_encoder();
+    if (!encode) return set_error(OB200_ERR_CUDA, "cannot resolve cuTensorMapEncodeTiled from the driver");
     static_assert(sizeof(BoardTensorMap) == sizeof(CUtensorMap), "tensor map size");
     if (((uintptr_t)base & 15) || rows <= 0 || box_rows <= 0 || box_rows > 256 || channels < kC || channels % kC)
         return set_error(OB200_ERR_INVALID,
@@ -329,6 +333,26 @@ int make_board_tensor_map(const void* base, long long rows, int box_rows, BoardT
                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(OB200_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+    return OB200_OK;
+}
+
+int make_board_plane_maps(const void* base, int S, int B, BoardPlaneMaps* out) {
+    const EncodeFn encode = tensor_map_encoder();
+    if (!encode) return set_error(OB200_ERR_CUDA, "cannot resolve cuTensorMapEncodeTiled from the driver");
+    if (((uintptr_t)base & 15) || S < 1 || S + 1 > 256 || B < 1)
+        return set_error(OB200_ERR_INVALID, "board plane map: base must be 16-byte aligned");
+    const int GP = S + 1;
+    for (int odd = 0; odd < 2; ++odd) {
+        const cuuint64_t dims[4] = {(cuuint64_t)kC, (cuuint64_t)((GP + 1 - odd) / 2), (cuuint64_t)GP, (cuuint64_t)B};
+        const cuuint64_t strides[3] = {2 * kRowBytes, (cuuint64_t)GP * kRowBytes, (cuuint64_t)GP * GP * kRowBytes};
+        const cuuint32_t box[4] = {(cuuint32_t)kC, (cuuint32_t)((GP + 1) / 2), (cuuint32_t)GP, 1};
+        const cuuint32_t estr[4] = {1, 1, 1, 1};
+        uint8_t* at = static_cast<uint8_t*>(const_cast<void*>(base)) + (size_t)(OB200_GUARD + odd) * kRowBytes;
+        const CUresult r = encode(reinterpret_cast<CUtensorMap*>(odd ? &out->odd : &out->even), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, at,
+                                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return set_error(OB200_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+    }
     return OB200_OK;
 }
 
