@@ -124,21 +124,6 @@ __device__ __forceinline__ int select_row(const ob200_tree_view& t, int node, fl
     return b.idx;
 }
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4)
-puct_select_kernel(ob200_tree_view t, const int32_t* __restrict__ node_ids, int n, float c_puct,
-                   int vl_value, int apply_vl, int32_t* __restrict__ sel_out) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const int node = node_ids ? node_ids[warp] : warp;
-    int sel = -1;
-    if (node >= 0 && node < t.n_nodes) sel = select_row<true>(t, node, c_puct, lane);
-    if (lane == 0) {
-        sel_out[warp] = sel;
-        if (sel >= 0 && apply_vl && vl_value > 0) atomicAdd(t.VL + (size_t)node * t.pitch + sel, vl_value);
-    }
-}
-
 // Cheap bracket of the score: one MUFU reciprocal per division instead of an IEEE
 // divide.  rcp.approx is within 1 ulp, so with q~ = val * rcp(ev), u~ = (p*explore) *
 // rcp(1 + ev) and m = |q~| + |u~| the exact score s (the reference's fp32 expression)
@@ -660,57 +645,79 @@ __global__ void vl_revert_kernel(ob200_tree_view t, const int32_t* __restrict__ 
     if (old < vl_value) atomicMax(addr, 0);
 }
 
+// One thread per edge of a path: every update is an atomic of its own and the value's sign is the parity of the
+// distance to the leaf, so the edges of a path need not wait for one another (a thread per path walked them one by one,
+// three trips to L2 each).
 __global__ void backup_kernel(ob200_tree_view t, const int32_t* __restrict__ paths,
                               const int32_t* __restrict__ path_len,
                               const float* __restrict__ leaf_values, int n, int max_depth,
                               int vl_value) {
     OB200_PDL_ENTER();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(idx / max_depth), d = (int)(idx - (long long)i * max_depth);
     if (i >= n) return;
-    int len = path_len[i];
-    if (len > max_depth) len = max_depth;
-    float v = leaf_values[i];
-    const int32_t* p = paths + (size_t)i * max_depth * 2;
-    for (int d = len - 1; d >= 0; --d) {
-        const int node = p[2 * d], s = p[2 * d + 1];
-        if (node < 0 || node >= t.n_nodes || s < 0 || s >= t.n_children) { v = -v; continue; }
-        const size_t e = (size_t)node * t.pitch + s;
-        atomicAdd(t.N + e, 1);
-        atomicAdd(t.W + e, v);
-        vl_sub_clamped(t.VL + e, vl_value, true);
-        if (d == len - 1 && t.child_node) {
-            const int child = t.child_node[e];
-            if (child >= 0 && child < t.n_nodes) atomicAdd(t.node_visits + child, 1);
-        }
-        atomicAdd(t.node_visits + node, 1);
-        v = -v;
+    // all of it before the first branch: it may come from host memory (ob200_tree_backup), one trip is enough
+    const int len = min(__ldcg(path_len + i), max_depth), node = __ldcg(paths + 2 * idx), s = __ldcg(paths + 2 * idx + 1);
+    const float leaf = __ldcg(leaf_values + i);
+    if (d >= len) return;
+    if (node < 0 || node >= t.n_nodes || s < 0 || s >= t.n_children) return;
+    const float v = ((len - 1 - d) & 1) ? -leaf : leaf;
+    const size_t e = (size_t)node * t.pitch + s;
+    atomicAdd(t.N + e, 1);
+    atomicAdd(t.W + e, v);
+    atomicAdd(t.node_visits + node, 1);
+    if (vl_value > 0) {
+        // update()'s unit and the revert's amount in one step: max(VL - 1 - amount, 0), as vl_revert_kernel does it
+        int32_t* vl = t.VL + e;
+        if (atomicSub(vl, vl_value + 1) < vl_value + 1) atomicMax(vl, 0);
+    } else vl_sub_clamped(t.VL + e, vl_value, true);
+    if (d == len - 1 && t.child_node) {
+        const int child = t.child_node[e];
+        if (child >= 0 && child < t.n_nodes) atomicAdd(t.node_visits + child, 1);
     }
 }
 
+// A warp per node; eight slots a lane are loaded before any is stored, so that a row of up to 256 slots costs one trip
+// to memory (the policy may be in host memory: ob200_tree_set_priors).
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 set_priors_kernel(ob200_tree_view t, const int32_t* __restrict__ node_ids, int n,
                   const float* __restrict__ policy, int policy_size,
                   const int32_t* __restrict__ slot_action) {
+    OB200_PDL_ENTER();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= n) return;
-    const int node = node_ids ? node_ids[warp] : warp;
-    if (node < 0 || node >= t.n_nodes) return;
-    const size_t row = (size_t)node * t.pitch;
-    const uint32_t* mask = t.legal_bits + (size_t)node * t.mask_words;
     const float* pol = policy + (size_t)warp * policy_size;
-    for (int s = lane; s < t.pitch; s += 32) {
-        float p = 0.0f;
-        if (s < t.n_children && ((mask[s >> 5] >> (s & 31)) & 1u)) {
-            const int a = slot_action ? slot_action[row + s] : s;
+    constexpr int kAhead = 8;
+    const int node = node_ids ? __ldcg(node_ids + warp) : warp;
+    for (int s0 = 0; s0 < t.pitch; s0 += 32 * kAhead) {
+        float p[kAhead];
+        uint32_t m[kAhead];
+        if (!slot_action)
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) p[k] = __ldcg(pol + min(s0 + k * 32 + lane, policy_size - 1));
+        if (node < 0 || node >= t.n_nodes) return;
+        const size_t row = (size_t)node * t.pitch;
+        const uint32_t* mask = t.legal_bits + (size_t)node * t.mask_words;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const int s = s0 + k * 32 + lane;
+            const bool in = s < t.n_children;
             // out-of-range actions get the reference's small default
-            p = (a >= 0 && a < policy_size) ? fminf(1.0f, fmaxf(0.0f, pol[a])) : 0.01f;
+            const int a = !in ? -1 : slot_action ? slot_action[row + s] : s;
+            if (a < 0 || a >= policy_size) p[k] = 0.01f;
+            else if (slot_action) p[k] = pol[a];
+            m[k] = in ? mask[s >> 5] >> (s & 31) : 0u;
         }
-        t.P[row + s] = p;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const int s = s0 + k * 32 + lane;
+            if (s < t.pitch) t.P[row + s] = (m[k] & 1u) ? fminf(1.0f, fmaxf(0.0f, p[k])) : 0.0f;
+        }
     }
 }
 
-// select_row for rows of at most 256 slots (two vectors a lane), as the descent uses it: approximate scores with one
+// select_row for rows of at most 256 slots (two vectors a lane), for the descent and small launches: approximate scores with one
 // error scale for the row, the exact expression only for the slots that can hold the maximum (see approx_score and
 // the segmented kernel above; the choice is the reference's bit for bit), instead of two IEEE divisions per slot.
 __device__ __forceinline__ int select_row_narrow(const ob200_tree_view& t, int node, float c_puct, int lane) {
@@ -768,6 +775,26 @@ __device__ __forceinline__ int select_row_narrow(const ob200_tree_view& t, int n
     if (b.idx < 0)
         return least_visited_row(t.N + row, mask, t.n_children, lane);
     return b.idx;
+}
+
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4)
+puct_select_kernel(ob200_tree_view t, const int32_t* __restrict__ node_ids, int n, float c_puct,
+                   int vl_value, int apply_vl, int32_t* __restrict__ sel_out) {
+    // the block's ids in one read and its results in one write: both may be in host memory (ob200_tree_select)
+    __shared__ int sel_s[kWarpsPerBlock];
+    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, first = blockIdx.x * kWarpsPerBlock;
+    int node = first + lane;
+    if (node_ids && lane < kWarpsPerBlock && node < n) node = node_ids[node];
+    node = __shfl_sync(0xffffffffu, node, wi);
+    int sel = -1;
+    if (first + wi < n && node >= 0 && node < t.n_nodes)
+        sel = t.pitch <= 256 ? select_row_narrow(t, node, c_puct, lane) : select_row<true>(t, node, c_puct, lane);
+    if (lane == 0) {
+        sel_s[wi] = sel;
+        if (sel >= 0 && apply_vl && vl_value > 0) atomicAdd(t.VL + (size_t)node * t.pitch + sel, vl_value);
+    }
+    __syncthreads();
+    if (threadIdx.x < kWarpsPerBlock && first + (int)threadIdx.x < n) sel_out[first + threadIdx.x] = sel_s[threadIdx.x];
 }
 
 // One CTA per tree.  Simulations of a tree are ordered: simulation k must see the virtual loss
@@ -995,7 +1022,7 @@ int ob200_launch_backup(const ob200_tree_view* tree, const int32_t* paths, const
         return set_error(OB200_ERR_INVALID, "ob200_launch_backup: bad arguments");
     if (int rc = require_device()) return rc;
     if (n == 0) return OB200_OK;
-    OB200_CUDA_OK(launch_dependent(backup_kernel, dim3((n + 127) / 128), dim3(128), 0, as_stream(stream), *tree, paths, path_len,
+    OB200_CUDA_OK(launch_dependent(backup_kernel, dim3((unsigned)(((long long)n * max_depth + 127) / 128)), dim3(128), 0, as_stream(stream), *tree, paths, path_len,
                                    leaf_values, n, max_depth, vl_value));
     counters().launches.fetch_add(1, std::memory_order_relaxed);
     counters().backups.fetch_add((uint64_t)n, std::memory_order_relaxed);
@@ -1011,9 +1038,9 @@ int ob200_launch_set_priors(const ob200_tree_view* tree, const int32_t* node_ids
     if (int rc = require_device()) return rc;
     if (n == 0) return OB200_OK;
     const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    set_priors_kernel<<<blocks, kWarpsPerBlock * 32, 0, as_stream(stream)>>>(*tree, node_ids, n, policy, policy_size,
-                                                                            slot_action);
-    OB200_LAUNCHED("set_priors_kernel");
+    OB200_CUDA_OK(launch_dependent(set_priors_kernel, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, as_stream(stream), *tree, node_ids, n, policy,
+                                   policy_size, slot_action));
+    counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
 }
 

@@ -3,8 +3,9 @@
 // setPriorProbabilities / expand (reference include/mcts/mcts_node.h:39-101, call sites
 // src/mcts/mcts_engine_batch_tree_simple.cpp:100-111,249-281), batched.  The edge statistics
 // live on the device as the structure of arrays of ob200_tree_view; arguments and results
-// cross the boundary through page-locked staging buffers owned by the handle, on its own
-// stream, one call at a time (internal mutex).
+// cross the boundary through page-locked memory owned by the handle, which the kernels read
+// and write in place: a call is one launch and one wait (10 us; a copy each way by the copy
+// engine is another 6).  On the handle's own stream, one call at a time (internal mutex).
 #include "internal.h"
 #include <algorithm>
 #include <cstring>
@@ -17,7 +18,8 @@ struct ob200_tree {
     ob200_tree_view view{};                    // device arrays; view.n_nodes = capacity
     cudaStream_t stream = nullptr;
     std::mutex mu;
-    // staging: one page-locked block and its device twin, grown on demand
+    // staging: one page-locked block at the same address on host and device, and a block of device memory for
+    // what large calls are better off copying; grown on demand
     unsigned char *h_stage = nullptr, *d_stage = nullptr;
     size_t stage_bytes = 0;
     std::vector<void*> owned;
@@ -37,14 +39,20 @@ int ensure_stage(ob200_tree* t, size_t bytes) {
     if (t->h_stage) cudaFreeHost(t->h_stage);
     if (t->d_stage) cudaFree(t->d_stage);
     t->h_stage = t->d_stage = nullptr; t->stage_bytes = 0;
-    OB200_CUDA_OK(cudaMallocHost(reinterpret_cast<void**>(&t->h_stage), want));
+    OB200_CUDA_OK(cudaHostAlloc(reinterpret_cast<void**>(&t->h_stage), want, cudaHostAllocPortable | cudaHostAllocMapped));
+    void* on_device = nullptr;
+    OB200_CUDA_OK(cudaHostGetDevicePointer(&on_device, t->h_stage, 0));
+    if (on_device != t->h_stage) return set_error(OB200_ERR_UNSUPPORTED, "tree: page-locked memory has another address on the device");
     OB200_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&t->d_stage), want));
     t->stage_bytes = want;
     return OB200_OK;
 }
 
-// Lays host arrays out in the staging block (256-byte aligned pieces), copies the block to the
-// device in one transfer and returns the device addresses.
+// Selections beyond this many nodes copy their ids and results: the kernels for large launches look ids up in the
+// middle of their row pipelines, where a trip to host memory would stall them, and write results four bytes at a time.
+constexpr int kSelectInPlace = 512;
+
+// Lays host arrays out in the staging block (256-byte aligned pieces).
 struct Stager {
     ob200_tree* t;
     size_t used = 0;
@@ -190,10 +198,9 @@ int ob200_tree_link(ob200_tree* t, int32_t n, const int32_t* parent, const int32
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, parent, (size_t)n * 4); std::memcpy(t->h_stage + b, slot, (size_t)n * 4);
     std::memcpy(t->h_stage + c, child, (size_t)n * 4);
-    OB200_CUDA_OK(cudaMemcpyAsync(t->d_stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
-    link_kernel<<<(n + 255) / 256, 256, 0, t->stream>>>(t->view, reinterpret_cast<int32_t*>(t->d_stage + a),
-                                                        reinterpret_cast<int32_t*>(t->d_stage + b),
-                                                        reinterpret_cast<int32_t*>(t->d_stage + c), n);
+    link_kernel<<<(n + 255) / 256, 256, 0, t->stream>>>(t->view, reinterpret_cast<int32_t*>(t->h_stage + a),
+                                                        reinterpret_cast<int32_t*>(t->h_stage + b),
+                                                        reinterpret_cast<int32_t*>(t->h_stage + c), n);
     OB200_LAUNCHED("link_kernel");
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     return OB200_OK;
@@ -210,10 +217,12 @@ int ob200_tree_select(ob200_tree* t, const int32_t* node_ids, int32_t n, float c
     const size_t a = s.reserve((size_t)n * 4), b = s.reserve((size_t)n * 4);
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, node_ids, (size_t)n * 4);
-    OB200_CUDA_OK(cudaMemcpyAsync(t->d_stage + a, t->h_stage + a, (size_t)n * 4, cudaMemcpyHostToDevice, t->stream));
-    if (int rc = ob200_launch_puct_select(&t->view, reinterpret_cast<int32_t*>(t->d_stage + a), n, c_puct, vl_value, apply_vl,
-                                          reinterpret_cast<int32_t*>(t->d_stage + b), t->stream)) return rc;
-    OB200_CUDA_OK(cudaMemcpyAsync(t->h_stage + b, t->d_stage + b, (size_t)n * 4, cudaMemcpyDeviceToHost, t->stream));
+    const bool in_place = n <= kSelectInPlace;
+    unsigned char* stage = in_place ? t->h_stage : t->d_stage;
+    if (!in_place) OB200_CUDA_OK(cudaMemcpyAsync(stage + a, t->h_stage + a, (size_t)n * 4, cudaMemcpyHostToDevice, t->stream));
+    if (int rc = ob200_launch_puct_select(&t->view, reinterpret_cast<int32_t*>(stage + a), n, c_puct, vl_value, apply_vl,
+                                          reinterpret_cast<int32_t*>(stage + b), t->stream)) return rc;
+    if (!in_place) OB200_CUDA_OK(cudaMemcpyAsync(t->h_stage + b, stage + b, (size_t)n * 4, cudaMemcpyDeviceToHost, t->stream));
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     std::memcpy(sel_out, t->h_stage + b, (size_t)n * 4);
     return OB200_OK;
@@ -231,9 +240,8 @@ int ob200_tree_virtual_loss(ob200_tree* t, const int32_t* node_ids, const int32_
     const size_t a = s.reserve((size_t)n * 4), b = s.reserve((size_t)n * 4);
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, node_ids, (size_t)n * 4); std::memcpy(t->h_stage + b, slots, (size_t)n * 4);
-    OB200_CUDA_OK(cudaMemcpyAsync(t->d_stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
-    const int32_t* dn = reinterpret_cast<int32_t*>(t->d_stage + a);
-    const int32_t* ds = reinterpret_cast<int32_t*>(t->d_stage + b);
+    const int32_t* dn = reinterpret_cast<int32_t*>(t->h_stage + a);
+    const int32_t* ds = reinterpret_cast<int32_t*>(t->h_stage + b);
     const int rc = amount > 0 ? ob200_launch_vl_apply(&t->view, dn, ds, n, amount, t->stream)
                               : ob200_launch_vl_revert(&t->view, dn, ds, n, -amount, t->stream);
     if (rc) return rc;
@@ -261,9 +269,8 @@ int ob200_tree_backup(ob200_tree* t, const int32_t* paths, const int32_t* path_l
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, paths, pb); std::memcpy(t->h_stage + b, path_len, (size_t)n * 4);
     std::memcpy(t->h_stage + c, leaf_values, (size_t)n * 4);
-    OB200_CUDA_OK(cudaMemcpyAsync(t->d_stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
-    if (int rc = ob200_launch_backup(&t->view, reinterpret_cast<int32_t*>(t->d_stage + a), reinterpret_cast<int32_t*>(t->d_stage + b),
-                                     reinterpret_cast<float*>(t->d_stage + c), n, max_depth, vl_value, t->stream)) return rc;
+    if (int rc = ob200_launch_backup(&t->view, reinterpret_cast<int32_t*>(t->h_stage + a), reinterpret_cast<int32_t*>(t->h_stage + b),
+                                     reinterpret_cast<float*>(t->h_stage + c), n, max_depth, vl_value, t->stream)) return rc;
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     return OB200_OK;
 }
@@ -278,8 +285,7 @@ int ob200_tree_set_priors(ob200_tree* t, const int32_t* node_ids, int32_t n, con
     const size_t a = s.reserve((size_t)n * 4), b = s.reserve((size_t)n * policy_size * 4);
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, node_ids, (size_t)n * 4); std::memcpy(t->h_stage + b, policy, (size_t)n * policy_size * 4);
-    OB200_CUDA_OK(cudaMemcpyAsync(t->d_stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
-    if (int rc = ob200_launch_set_priors(&t->view, reinterpret_cast<int32_t*>(t->d_stage + a), n, reinterpret_cast<float*>(t->d_stage + b),
+    if (int rc = ob200_launch_set_priors(&t->view, reinterpret_cast<int32_t*>(t->h_stage + a), n, reinterpret_cast<float*>(t->h_stage + b),
                                          policy_size, nullptr, t->stream)) return rc;
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     return OB200_OK;
