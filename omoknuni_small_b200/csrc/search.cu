@@ -52,7 +52,8 @@ struct ob200_search {
     uint64_t gamma_for = 0;
     uint32_t* empty_bits = nullptr;            // [max_nodes][mask_words], only when a node's children can be fewer than its legal moves
     int max_children = 1000, widen_target = 0;
-    // expansion plan of a round (per simulation)
+    // a round's leaf edges (node, slot; node -1: the root itself is the leaf) and its expansion plan (per simulation)
+    int2* leaf_edge = nullptr;
     int32_t *plan_status = nullptr, *plan_aux = nullptr, *plan_new_id = nullptr;
     unsigned long long* plan_hash = nullptr;
     // test hooks: leaf values rounded to multiples of 1 / value_quantum (0 = off); a record of what every network
@@ -118,66 +119,93 @@ __global__ void mix_noise_kernel(ob200_tree_view t, const float* __restrict__ no
             t.P[row + s] = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, eps), t.P[row + s]), __fmul_rn(eps, noise[(size_t)tree * t.pitch + s]));
 }
 
-// One thread per simulation: the leaf position from root + path.
+// One warp per simulation: the leaf position from root + path.
 //   history (k-th most recent move), side to move, and whether the game is over:
 //   five or more in a row through the last move for the player who made it
 //   (freestyle rules), or a full board.
-__global__ void leaf_prepare_kernel(const int32_t* __restrict__ paths, const int32_t* __restrict__ path_len,
-                                    int n_sims, int sims_per_tree, int max_depth, int S,
-                                    const uint32_t* __restrict__ root_stones, const int16_t* __restrict__ root_hist,
-                                    const uint8_t* __restrict__ root_nh, const uint8_t* __restrict__ root_tm,
-                                    const int32_t* __restrict__ root_count, int16_t* __restrict__ leaf_hist,
-                                    uint8_t* __restrict__ leaf_nh, uint8_t* __restrict__ leaf_tm,
-                                    float* __restrict__ term_value, int32_t* term_count, int rules) {
+// And what the expansion needs to know of the leaf edge: (node, slot), and the key of the position behind it.
+// Everything is loaded at once, one element a lane (two of the path), and taken apart with shuffles: one trip to L2
+// and one for the parent's key, where a thread per simulation walked path and lines one load at a time (8.5 us; now
+// 4.5, measured cold).
+struct LeafOut {
+    int16_t* hist; uint8_t *nh, *tm;
+    float* term_value; int32_t* term_count;
+    int2* edge; unsigned long long* hash;
+};
+__global__ void __launch_bounds__(128)
+leaf_prepare_kernel(const int32_t* __restrict__ paths, const int32_t* __restrict__ path_len,
+                    int n_sims, int sims_per_tree, int max_depth, int S,
+                    const uint32_t* __restrict__ root_stones, const int16_t* __restrict__ root_hist,
+                    const uint8_t* __restrict__ root_nh, const uint8_t* __restrict__ root_tm,
+                    const int32_t* __restrict__ root_count, int rules, const unsigned long long* __restrict__ zobrist,
+                    const unsigned long long* __restrict__ node_hash, const LeafOut out) {
     OB200_PDL_ENTER();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n_sims) return;
     const int tree = i / sims_per_tree;
-    int len = path_len[i];
-    if (len > max_depth) len = max_depth;
-    const int32_t* p = paths + (size_t)i * max_depth * 2;
-    const int rtm = root_tm[tree], rnh = root_nh[tree];
+    const int2* p = reinterpret_cast<const int2*>(paths) + (size_t)i * max_depth;
+    const int len = min(path_len[i], max_depth);
+    const int2 step0 = lane < max_depth ? __ldcg(p + lane) : make_int2(-1, -1);
+    const int2 step1 = lane + 32 < max_depth ? __ldcg(p + lane + 32) : make_int2(-1, -1);
+    const int rtm = root_tm[tree], rnh = root_nh[tree], rcount = root_count[tree];
+    const int rhist = lane < 16 ? root_hist[(size_t)tree * 16 + lane] : -1;
+    const uint32_t rstones = lane < 16 ? root_stones[(size_t)tree * 16 + lane] : 0u;
+    auto slot_at = [&](int d) {          // the move at depth d (any lane's own d)
+        const int a = __shfl_sync(0xffffffffu, step0.y, d & 31), b = __shfl_sync(0xffffffffu, step1.y, d & 31);
+        return d < 32 ? a : b;
+    };
     const int tm = (len & 1) ? 3 - rtm : rtm;
-    int nh = 0;
-    for (int k = 0; k < 16; ++k) {
-        int mv = -1;
-        if (k < len) mv = p[2 * (len - 1 - k) + 1];
-        else if (k - len < rnh) mv = root_hist[(size_t)tree * 16 + (k - len)];
-        leaf_hist[(size_t)i * 16 + k] = (int16_t)mv;
-        if (mv >= 0) nh = k + 1;
-    }
-    leaf_nh[i] = (uint8_t)nh;
-    leaf_tm[i] = (uint8_t)tm;
+    // history: lane k < 16 holds the k-th most recent move
+    const int from_path = slot_at(max(len - 1 - lane, 0)), from_root = __shfl_sync(0xffffffffu, rhist, (lane - len) & 31);
+    const int mv = lane < len ? from_path : lane - len < rnh ? from_root : -1;
+    const uint32_t have = __ballot_sync(0xffffffffu, lane < 16 && mv >= 0);
+    if (lane < 16) out.hist[(size_t)i * 16 + lane] = (int16_t)mv;
+    if (lane == 0) { out.nh[i] = (uint8_t)(32 - __clz(have)); out.tm[i] = (uint8_t)tm; }
     float tv = nanf("");
     if (len > 0) {
+        const int parent_a = __shfl_sync(0xffffffffu, step0.x, (len - 1) & 31), parent_b = __shfl_sync(0xffffffffu, step1.x, (len - 1) & 31);
+        const int parent = len - 1 < 32 ? parent_a : parent_b, last = slot_at(len - 1);
         const int mover = 3 - tm;                              // who made the last move
-        const uint32_t* st = root_stones + (size_t)tree * 16 + (mover - 1) * 8;
-        const int last = p[2 * (len - 1) + 1];
+        unsigned long long key = 0;
+        if (lane == 0 && zobrist) key = node_hash[parent] ^ zobrist[(mover - 1) * 225 + last] ^ zobrist[450];
+        // the mover's stones, a word in each of the lanes 0-7: the root's and every second move of the path
+        uint32_t own = __shfl_sync(0xffffffffu, rstones, (mover - 1) * 8 + (lane & 7));
+        for (int d = len - 1; d >= 0; d -= 2) {
+            const int a = slot_at(d);
+            if (lane == (a >> 5)) own |= 1u << (a & 31);
+        }
+        // lanes 8 dir + k - 1: is the k-th cell (k = 1..5) along the direction the mover's?
+        const int dir = lane >> 3, k = (lane & 7) + 1;
+        const int dr = dir == 0 ? 0 : 1, dc = dir == 1 ? 0 : dir == 3 ? -1 : 1;
         const int r0 = last / S, c0 = last % S;
-        auto has = [&](int r, int c) {
-            if (r < 0 || r >= S || c < 0 || c >= S) return false;
-            const int cell = r * S + c;
-            if (bit(st, cell)) return true;
-            for (int d = len - 1; d >= 0; d -= 2)              // the mover's moves on the path
-                if (p[2 * d + 1] == cell) return true;
-            return false;
+        auto line = [&](int sign) {
+            const int r = r0 + sign * k * dr, c = c0 + sign * k * dc;
+            const bool in = k <= 5 && r >= 0 && r < S && c >= 0 && c < S;
+            const int cell = in ? r * S + c : 0;
+            const uint32_t word = __shfl_sync(0xffffffffu, own, cell >> 5);
+            return __ballot_sync(0xffffffffu, in && ((word >> (cell & 31)) & 1u));
         };
-        const int dr[4] = {0, 1, 1, 1}, dc[4] = {1, 0, 1, -1};
+        const uint32_t fwd = line(1), back = line(-1);
         // five or more wins; under Renju BLACK needs exactly five and no longer line through the stone
         // (GomokuState::refresh_winner_cache, src/games/gomoku/gomoku_state.cpp:812-860)
         bool five_up = false, exact = false, over = false;
-        for (int dir = 0; dir < 4; ++dir) {
-            int run = 1;
-            for (int k = 1; k < 6 && has(r0 + k * dr[dir], c0 + k * dc[dir]); ++k) ++run;
-            for (int k = 1; k < 6 && has(r0 - k * dr[dir], c0 - k * dc[dir]); ++k) ++run;
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            const int run = 1 + (__ffs(~((fwd >> (8 * d)) & 0x1Fu)) - 1) + (__ffs(~((back >> (8 * d)) & 0x1Fu)) - 1);
             five_up = five_up || run >= 5; exact = exact || run == 5; over = over || run > 5;
         }
         const bool win = (rules == OB200_RULES_RENJU && mover == 1) ? (exact && !over) : five_up;
         if (win) tv = -1.0f;                                    // the side to move has lost
-        else if (root_count[tree] + len >= S * S) tv = 0.0f;    // full board
+        else if (rcount + len >= S * S) tv = 0.0f;              // full board
+        if (lane == 0) {
+            out.edge[i] = make_int2(parent, last);
+            if (zobrist) out.hash[i] = key ? key : 1ull;
+        }
+    } else if (lane == 0) out.edge[i] = make_int2(-1, -1);
+    if (lane == 0) {
+        out.term_value[i] = tv;
+        if (tv == tv) atomicAdd(out.term_count, 1);
     }
-    term_value[i] = tv;
-    if (tv == tv) atomicAdd(term_count, 1);
 }
 
 // Expansion of a round's leaf edges, in two kernels.  The outcome is a function of the inputs alone
@@ -199,6 +227,11 @@ __global__ void leaf_prepare_kernel(const int32_t* __restrict__ paths, const int
 //      per key becomes its owner;
 //   D  owners are counted in index order (block scan) -> node ids;
 //   E  edges and table entries are pointed at the ids.
+// expand_plan_small_kernel does the same for rounds of up to 1,024 simulations with a thread per simulation, whose
+// state stays in registers; who owns an edge or a key is settled in two hash tables in shared memory instead of by
+// atomics on the edges and the table's values, and the table is looked up while the edges are still on their way: four
+// trips to L2 instead of a dozen (with the leaf and row kernels below, which were taken apart the same way: a round of
+// 16 simulations 9 us shorter, one of 1,024 also 9 us).
 // expand_rows_kernel (a warp per simulation) then fills the rows of the nodes created.
 constexpr int kPlanThreads = 1024;
 enum : int32_t { kPlanNone = 0, kPlanCandidate = 1, kPlanNew = 2, kPlanShareOld = 3, kPlanShareNew = 4, kPlanOwner = 5 };
@@ -331,33 +364,160 @@ expand_plan_kernel(ob200_tree_view t, const int32_t* __restrict__ paths, const i
     }
 }
 
+// Open addressing in shared memory: the lowest index that enters a key.  Twice as many slots as simulations.
+constexpr int kPlanSlots = 2 * kPlanThreads;
+struct PlanTable {
+    unsigned long long key[kPlanSlots];      // 0: free
+    int lowest[kPlanSlots];
+    __device__ void clear(int tid) {
+        for (int i = tid; i < kPlanSlots; i += kPlanThreads) { key[i] = 0ull; lowest[i] = INT_MAX; }
+    }
+    __device__ int enter(unsigned long long k, int index) {      // returns the key's slot
+        unsigned at = (unsigned)((k * 0x9E3779B97F4A7C15ull) >> 40) & (kPlanSlots - 1);
+        for (;; at = (at + 1) & (kPlanSlots - 1)) {              // ends: there are more slots than keys
+            const unsigned long long seen = atomicCAS(&key[at], 0ull, k);
+            if (seen == 0ull || seen == k) break;
+        }
+        atomicMin(&lowest[at], index);
+        return (int)at;
+    }
+};
+struct PlanShared {
+    PlanTable edges, keys;
+    int new_id[kPlanThreads];
+    uint8_t in_table[kPlanThreads];
+    int warp_sums[kPlanThreads / 32];
+};
+
+__global__ void __launch_bounds__(kPlanThreads)
+expand_plan_small_kernel(ob200_tree_view t, const int2* __restrict__ edges, const unsigned long long* __restrict__ hashes, int n_sims,
+                         const float* __restrict__ value, const float* __restrict__ term_value, float value_sign, float value_quantum,
+                         int max_nodes, int32_t* n_used, float* __restrict__ leaf_value, unsigned long long* tt_key, int32_t* tt_val,
+                         int tt_size, int32_t* __restrict__ new_id_out) {
+    extern __shared__ __align__(16) uint8_t plan_smem[];
+    PlanShared& sh = *reinterpret_cast<PlanShared*>(plan_smem);
+    const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+    sh.edges.clear(i);
+    sh.keys.clear(i);
+    sh.in_table[i] = 1;
+    OB200_PDL_ENTER();
+    const bool mine = i < n_sims;
+    const int2 edge = mine ? __ldcg(edges + i) : make_int2(-1, -1);
+    const float tv = mine ? term_value[i] : 0.0f, nv = mine ? value[i] : 0.0f;
+    const unsigned long long h = mine && tt_size > 0 && edge.x >= 0 ? __ldcg(hashes + i) : 1ull;
+    const int base = *n_used;
+    const bool terminal = tv == tv;
+    if (mine) leaf_value[i] = value_sign * (terminal ? tv : quantized(nv, value_quantum));
+    const bool leaf = mine && edge.x >= 0 && !terminal;
+    const size_t e = leaf ? (size_t)edge.x * t.pitch + edge.y : 0;
+    // the edge's child and the key's first table entry in one trip
+    unsigned idx = (unsigned)(h >> 17) & (unsigned)(tt_size - 1);
+    const int child_before = leaf ? __ldcg(t.child_node + e) : 0;
+    unsigned long long k = leaf && tt_size > 0 ? __ldcg(tt_key + idx) : 0ull;
+    int st = leaf && child_before < 0 ? kPlanCandidate : kPlanNone, slot = -1, share = -1;
+    __syncthreads();
+    // ---- A: the lowest index per edge ----
+    if (st == kPlanCandidate) slot = sh.edges.enter((unsigned long long)e + 1ull, i);
+    __syncthreads();
+    if (st == kPlanCandidate && sh.edges.lowest[slot] != i) st = kPlanNone;
+    // ---- B: winners; table lookup against the state before this round ----
+    slot = -1;
+    if (st == kPlanCandidate) {
+        st = kPlanNew;                                                    // no table, or probe limit reached: a node outside it
+        if (tt_size > 0)
+            for (int tries = 0;;) {
+                if (k == 0) { st = kPlanCandidate; break; }
+                if (k == h) {
+                    share = __ldcg(tt_val + idx);
+                    st = share >= 0 ? kPlanShareOld : kPlanCandidate;
+                    break;
+                }
+                if (++tries == 64) break;
+                idx = (idx + 1) & (unsigned)(tt_size - 1);
+                k = __ldcg(tt_key + idx);
+            }
+        // the lowest index per key among this round's new positions
+        if (st == kPlanCandidate) slot = sh.keys.enter(h, i);
+    }
+    __syncthreads();
+    // ---- C: owners enter their key ----
+    int owner = i, found = -1;
+    if (st == kPlanCandidate) {
+        owner = sh.keys.lowest[slot];
+        if (owner == i) {
+            idx = (unsigned)(h >> 17) & (unsigned)(tt_size - 1);
+            for (int tries = 0; tries < 64 && found < 0; ++tries, idx = (idx + 1) & (unsigned)(tt_size - 1)) {
+                const unsigned long long seen = atomicCAS(tt_key + idx, 0ull, h);
+                if (seen == 0ull || seen == h) found = (int)idx;
+            }
+            if (found < 0) sh.in_table[i] = 0;
+        }
+    }
+    __syncthreads();
+    if (st == kPlanCandidate) {
+        // a key that found no place in the table leaves each of its simulations a node of its own
+        st = !sh.in_table[owner] ? kPlanNew : owner == i ? kPlanOwner : kPlanShareNew;
+    }
+    // ---- D: ids in index order ----
+    const int flag = (st == kPlanOwner || st == kPlanNew) ? 1 : 0;
+    const uint32_t votes = __ballot_sync(0xffffffffu, flag);
+    if (lane == 0) sh.warp_sums[warp] = __popc(votes);
+    __syncthreads();
+    if (warp == 0) {
+        int w = sh.warp_sums[lane];
+        for (int off = 1; off < 32; off <<= 1) { const int o = __shfl_up_sync(0xffffffffu, w, off); if (lane >= off) w += o; }
+        sh.warp_sums[lane] = w;                                           // inclusive sums over the warps
+    }
+    __syncthreads();
+    const int before = base + (warp ? sh.warp_sums[warp - 1] : 0) + __popc(votes & ((1u << lane) - 1u));
+    const int id = flag && before < max_nodes ? before : -1;             // pool exhausted: the edge stays a leaf
+    sh.new_id[i] = id;
+    if (mine) new_id_out[i] = id;
+    if (i == 0) { const int used = base + sh.warp_sums[kPlanThreads / 32 - 1]; *n_used = used < max_nodes ? used : max_nodes; }
+    __syncthreads();
+    // ---- E: point edges and table entries at the nodes ----
+    if (st == kPlanNone) return;
+    if (st == kPlanOwner) tt_val[found] = id;
+    t.child_node[e] = st == kPlanShareOld ? share : st == kPlanShareNew ? sh.new_id[owner] : id;
+}
+
 // One warp per simulation that creates a node: existence mask = the parent's minus the move, priors =
 // clamp(policy, 0, 1) on the existing slots with no renormalisation (MCTSNode::expand +
-// setPriorProbabilities, src/mcts/mcts_node.cpp:238-436,546-553), statistics zero.
+// setPriorProbabilities, src/mcts/mcts_node.cpp:238-436,546-553), statistics zero.  Rows of at most 256 slots.
 __global__ void __launch_bounds__(256)
 expand_rows_kernel(ob200_tree_view t, const int32_t* __restrict__ paths, const int32_t* __restrict__ path_len,
                    int n_sims, int max_depth, const float* __restrict__ policy, int policy_size,
-                   unsigned long long* node_hash, int tt_size, PlanScratch ps, Widening wd,
+                   unsigned long long* node_hash, int tt_size, const int32_t* __restrict__ new_id,
+                   const int2* __restrict__ edges, const unsigned long long* __restrict__ hashes, Widening wd,
                    const uint32_t* __restrict__ root_stones, const uint8_t* __restrict__ root_tm, int sims_per_tree, int S) {
     __shared__ uint32_t black_s[8][8], legal_s[8][8];
     OB200_PDL_ENTER();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     if (i >= n_sims) return;
-    const int st = ps.status[i];
-    const int id = ps.new_id[i];
-    if ((st != kPlanOwner && st != kPlanNew) || id < 0) return;
-    int len = path_len[i];
-    if (len > max_depth) len = max_depth;
-    const int32_t* p = paths + (size_t)i * max_depth * 2;
-    const int parent = p[2 * (len - 1)], slot = p[2 * (len - 1) + 1];
+    // the policy row comes along with the ids, whether there is a node to fill or not: one trip less
+    constexpr int kAhead = 8;
+    float pol[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) pol[k] = __ldcg(policy + (size_t)i * policy_size + min(k * 32 + lane, policy_size - 1));
+    const int id = __ldcg(new_id + i);
+    const int2 edge = __ldcg(edges + i);
+    const unsigned long long h = tt_size > 0 ? __ldcg(hashes + i) : 0ull;
+    if (id < 0) return;
+    const int parent = edge.x, slot = edge.y;
     const size_t row = (size_t)id * t.pitch;
     // the position's empty cells: the parent's minus the move; they are the children unless the node is widened
     const uint32_t* pm = (wd.empty ? wd.empty : t.legal_bits) + (size_t)parent * t.mask_words;
     uint32_t* own = (wd.empty ? wd.empty : t.legal_bits) + (size_t)id * t.mask_words;
     uint32_t* cm = t.legal_bits + (size_t)id * t.mask_words;
-    for (int w = lane; w < t.mask_words; w += 32) own[w] = pm[w] & ~((w == (slot >> 5)) ? (1u << (slot & 31)) : 0u);
+    uint32_t word = 0u;
+    if (lane < t.mask_words) {
+        word = pm[lane] & ~((lane == (slot >> 5)) ? (1u << (slot & 31)) : 0u);
+        own[lane] = word;
+    }
     __syncwarp();
     if (wd.empty) {
+        const int len = min(path_len[i], max_depth);
+        const int32_t* p = paths + (size_t)i * max_depth * 2;
         const int tree = i / sims_per_tree;
         const bool black_to_move = (root_tm[tree] == 1) == ((len & 1) == 0);     // the root's side moves at even depths
         if (wd.rules != OB200_RULES_FREESTYLE && black_to_move) {
@@ -374,17 +534,20 @@ expand_rows_kernel(ob200_tree_view t, const int32_t* __restrict__ paths, const i
         legal_moves_warp(black_s[wi], own, legal_s[wi], S, t.mask_words, wd.rules, black_to_move, lane);
         widen_mask_warp(legal_s[wi], cm, t.mask_words, wd, id, lane);
         __syncwarp();
+        if (lane < t.mask_words) word = cm[lane];
     }
-    const float* pol = policy + (size_t)i * policy_size;
-    for (int s = lane; s < t.pitch; s += 32) {
-        float pr = 0.0f;
-        if (s < t.n_children && bit(cm, s)) pr = fminf(1.0f, fmaxf(0.0f, pol[s]));
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+        const int s = k * 32 + lane;
+        const uint32_t m = __shfl_sync(0xffffffffu, word, k);
+        if (s >= t.pitch) continue;
+        const float pr = s < t.n_children && ((m >> lane) & 1u) ? fminf(1.0f, fmaxf(0.0f, pol[k])) : 0.0f;
         t.N[row + s] = 0; t.W[row + s] = 0.0f; t.VL[row + s] = 0; t.P[row + s] = pr;
         t.child_node[row + s] = -1;
     }
     if (lane == 0) {
         t.node_visits[id] = 0;
-        if (tt_size > 0) node_hash[id] = ps.hash[i];
+        if (tt_size > 0) node_hash[id] = h;
     }
 }
 
@@ -471,7 +634,7 @@ int ob200_search_create(ob200_net* net, const ob200_search_config* cfg, ob200_se
     A_(salloc(s, &s->policy, (size_t)L * s->A)); A_(salloc(s, &s->value, (size_t)L));
     A_(salloc(s, &s->noise, (size_t)T * s->pitch));
     A_(salloc(s, &s->plan_status, (size_t)L)); A_(salloc(s, &s->plan_aux, (size_t)L)); A_(salloc(s, &s->plan_new_id, (size_t)L));
-    A_(salloc(s, &s->plan_hash, (size_t)L));
+    A_(salloc(s, &s->plan_hash, (size_t)L)); A_(salloc(s, &s->leaf_edge, (size_t)L));
     if (cfg->use_transposition_table) {
         s->tt_size = 1;
         while (s->tt_size < 2 * s->max_nodes) s->tt_size <<= 1;
@@ -494,6 +657,7 @@ int ob200_search_create(ob200_net* net, const ob200_search_config* cfg, ob200_se
         }
         OB200_CUDA_OK(cudaMemcpy(s->zobrist, s->zobrist_host.data(), 451 * 8, cudaMemcpyHostToDevice));
     }
+    OB200_CUDA_OK(cudaFuncSetAttribute(expand_plan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PlanShared)));
     OB200_CUDA_OK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     OB200_CUDA_OK(cudaEventCreate(&s->ev0)); OB200_CUDA_OK(cudaEventCreate(&s->ev1));
     *out = s;
@@ -656,9 +820,10 @@ int ob200_search_run(ob200_search* s, const int16_t* moves, const int32_t* n_mov
         if (int rc = ob200_launch_traverse(&s->tv, s->roots, T, s->sims_per_round, c.c_puct, c.virtual_loss, c.max_depth,
                                            s->paths, s->path_len, st)) return rc;
         OB200_CUDA_OK(mark(r, 1));
-        OB200_CUDA_OK(launch_dependent(leaf_prepare_kernel, dim3((L + 127) / 128), dim3(128), 0, st, s->paths, s->path_len, L,
+        const LeafOut leaf{s->leaf_hist, s->leaf_nh, s->leaf_tm, s->term_value, s->term_count, s->leaf_edge, s->plan_hash};
+        OB200_CUDA_OK(launch_dependent(leaf_prepare_kernel, dim3((L + 3) / 4), dim3(128), 0, st, s->paths, s->path_len, L,
                                        s->sims_per_round, c.max_depth, S, s->root_stones, s->root_hist, s->root_nh, s->root_tm,
-                                       s->root_count, s->leaf_hist, s->leaf_nh, s->leaf_tm, s->term_value, s->term_count, c.rules));
+                                       s->root_count, c.rules, s->zobrist, s->node_hash, leaf));
         counters().launches.fetch_add(1, std::memory_order_relaxed);
         OB200_CUDA_OK(mark(r, 2));
         if (int rc = net_forward_gomoku_for_search(s->net, s->leaf_hist, s->leaf_nh, s->leaf_tm, L, s->policy, s->value, st)) return rc;
@@ -667,14 +832,20 @@ int ob200_search_run(ob200_search* s, const int16_t* moves, const int32_t* n_mov
             OB200_CUDA_OK(cudaMemcpyAsync(s->rec_policy + (size_t)(r + 1) * L * A, s->policy, (size_t)L * A * 4, cudaMemcpyDeviceToDevice, st));
             OB200_CUDA_OK(cudaMemcpyAsync(s->rec_value + (size_t)(r + 1) * L, s->value, (size_t)L * 4, cudaMemcpyDeviceToDevice, st));
         }
-        const PlanScratch ps{s->plan_status, s->plan_aux, s->plan_new_id, s->plan_hash};
-        OB200_CUDA_OK(launch_dependent(expand_plan_kernel, dim3(1), dim3(kPlanThreads), 0, st, s->tv, s->paths, s->path_len, L, c.max_depth,
-                                       s->value, s->term_value, (float)c.value_sign, s->value_quantum, s->max_nodes, s->n_used,
-                                       s->leaf_value, s->sims_per_round, s->root_tm, s->zobrist, s->node_hash, s->tt_key, s->tt_val,
-                                       s->tt_size, ps));
+        if (L <= kPlanThreads) {
+            OB200_CUDA_OK(launch_dependent(expand_plan_small_kernel, dim3(1), dim3(kPlanThreads), sizeof(PlanShared), st, s->tv, s->leaf_edge,
+                                           s->plan_hash, L, s->value, s->term_value, (float)c.value_sign, s->value_quantum, s->max_nodes,
+                                           s->n_used, s->leaf_value, s->tt_key, s->tt_val, s->tt_size, s->plan_new_id));
+        } else {
+            const PlanScratch ps{s->plan_status, s->plan_aux, s->plan_new_id, s->plan_hash};
+            OB200_CUDA_OK(launch_dependent(expand_plan_kernel, dim3(1), dim3(kPlanThreads), 0, st, s->tv, s->paths, s->path_len, L, c.max_depth,
+                                           s->value, s->term_value, (float)c.value_sign, s->value_quantum, s->max_nodes, s->n_used,
+                                           s->leaf_value, s->sims_per_round, s->root_tm, s->zobrist, s->node_hash, s->tt_key, s->tt_val,
+                                           s->tt_size, ps));
+        }
         OB200_CUDA_OK(launch_dependent(expand_rows_kernel, dim3((L * 32 + 255) / 256), dim3(256), 0, st, s->tv, s->paths, s->path_len, L,
-                                       c.max_depth, s->policy, A, s->node_hash, s->tt_size, ps, wd, s->root_stones, s->root_tm,
-                                       s->sims_per_round, s->S));
+                                       c.max_depth, s->policy, A, s->node_hash, s->tt_size, s->plan_new_id, s->leaf_edge, s->plan_hash, wd,
+                                       s->root_stones, s->root_tm, s->sims_per_round, s->S));
         counters().launches.fetch_add(2, std::memory_order_relaxed);
         OB200_CUDA_OK(mark(r, 4));
         if (int rc = ob200_launch_backup(&s->tv, s->paths, s->path_len, s->leaf_value, L, c.max_depth, c.virtual_loss, st)) return rc;

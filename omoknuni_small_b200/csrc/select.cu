@@ -155,6 +155,13 @@ __device__ __forceinline__ void bracket(int n, float w, float p, int vl, float e
     hi = legal ? fmaf(kBracket, m, s) : -INFINITY;
 }
 
+// Maximum over the warp; NaNs are ignored, as fmaxf ignores them.
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 constexpr int kWideMinPitch = 1024;          // rows at least this wide always take the segmented kernel
 constexpr long long kSegMinItems = 24576;    // narrower rows (257-1,023 slots) take it from this many segments on
 
@@ -293,8 +300,7 @@ puct_select_staged_kernel(ob200_tree_view t, const int32_t* __restrict__ node_id
                 bracket(nn.z, ww.z, pp.z, ll.z, explore, m & 4u, lo, hi[4 * h + 2]); lane_lo = fmaxf(lane_lo, lo);
                 bracket(nn.w, ww.w, pp.w, ll.w, explore, m & 8u, lo, hi[4 * h + 3]); lane_lo = fmaxf(lane_lo, lo);
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) lane_lo = fmaxf(lane_lo, __shfl_xor_sync(0xffffffffu, lane_lo, off));
+            lane_lo = warp_max(lane_lo);
             // pass 2: the slots whose bracket reaches the best lower bound.  Usually there is
             // exactly one, and with a finite bound it is the answer without any exact score.
             uint32_t cand = 0;
@@ -519,11 +525,8 @@ puct_select_segmented_kernel(ob200_tree_view t, const int32_t* __restrict__ node
             lane_s = -INFINITY; lane_m = 0.0f;
             scores(std::false_type{});
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            lane_s = fmaxf(lane_s, __shfl_xor_sync(0xffffffffu, lane_s, off));
-            lane_m = fmaxf(lane_m, __shfl_xor_sync(0xffffffffu, lane_m, off));
-        }
+        lane_s = warp_max(lane_s);
+        lane_m = warp_max(lane_m);
         float thr = fmaf(-2.0f * kBracket, lane_m, lane_s);
         thr = thr == thr ? thr : -INFINITY;       // inf - inf: no usable bound, every existing slot is a candidate
         uint32_t cand = 0;
@@ -757,17 +760,28 @@ __device__ __forceinline__ int select_row_narrow(const ob200_tree_view& t, int n
 #pragma unroll
         for (int k = 0; k < 8; ++k) approx_score<false>(n8[k], w8[k], p8[k], l8[k], explore, (bits >> k) & 1u, sc[k], lane_s, lane_m, range);
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        lane_s = fmaxf(lane_s, __shfl_xor_sync(0xffffffffu, lane_s, off));
-        lane_m = fmaxf(lane_m, __shfl_xor_sync(0xffffffffu, lane_m, off));
-    }
+    lane_s = warp_max(lane_s);
+    lane_m = warp_max(lane_m);
     float thr = fmaf(-2.0f * kBracket, lane_m, lane_s);
     thr = thr == thr ? thr : -INFINITY;
+    uint32_t cand = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) cand |= (uint32_t)(sc[k] >= thr) << k;
+    cand &= bits;
+    // Nearly always one slot is left.  With a finite bound its exact score is finite too, so it is the choice.
+    const uint32_t lanes = __ballot_sync(0xffffffffu, cand != 0);
+    if (__popc(lanes) == 1 && lane_s > -INFINITY) {
+        const int l = __ffs(lanes) - 1;
+        const uint32_t c = __shfl_sync(0xffffffffu, cand, l);
+        if (!(c & (c - 1))) {
+            const int k = __ffs(c) - 1;
+            return (l + 32 * (k >> 2)) * 4 + (k & 3);
+        }
+    }
     Best b{-INFINITY, -1};
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        if (((bits >> k) & 1u) && sc[k] >= thr) {
+        if ((cand >> k) & 1u) {
             const float e = puct_score(n8[k], w8[k], p8[k], l8[k], explore);
             if (e > b.score) { b.score = e; b.idx = (lane + 32 * (k >> 2)) * 4 + (k & 3); }
         }
