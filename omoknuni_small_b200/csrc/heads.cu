@@ -177,10 +177,11 @@ constexpr int kTailRegs = 2;             // logits a thread keeps in registers: 
 __global__ void __launch_bounds__(kTailThreads)
 head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __restrict__ logits, int A, int policy_rows, int softmax,
                   const HeadFcLayer val, const float* __restrict__ b1, const float* __restrict__ w2, float b2, int H, int B,
-                  float* __restrict__ value) {
+                  float* __restrict__ value, const int* error_word, int* error_out) {
     __shared__ float red[kTailThreads / 32];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (error_out && blockIdx.x == 0 && threadIdx.x == 0) *error_out = __ldcg(error_word);
     if ((int)blockIdx.x < policy_rows) {
         const int b = blockIdx.x;
         float* row = logits + (size_t)b * A;
@@ -235,10 +236,11 @@ head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __
 
 int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_out, int policy_size, int softmax,
                       const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
-                      cudaStream_t st) {
+                      cudaStream_t st, int* error_out) {
     const int rows = policy_out && (policy.part || softmax) ? B : 0;
     OB200_CUDA_OK(launch_dependent(head_tails_kernel, dim3((unsigned)(rows + B)), dim3(kTailThreads), 0, st, policy, bp,
-                                   policy_out, policy_size, rows, softmax, value, b1, w2, b2, H, B, value_out));
+                                   policy_out, policy_size, rows, softmax, value, b1, w2, b2, H, B, value_out,
+                                   (const int*)(error_out ? device_error_word() : nullptr), error_out));
     counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
 }

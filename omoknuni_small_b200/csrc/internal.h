@@ -87,9 +87,10 @@ int head_fc_plan(HeadFcLayer* l, int n_layers, int B, int sms);
 int launch_head_fc(const HeadFcLayer* layers, int n_layers, int B, cudaStream_t st);
 // What is left of both heads in one launch: partial sums + bias -> logits (or softmax of them), partial sums + bias ->
 // ReLU -> value FC2 -> tanh.  policy.part may be null: the logits are in policy_out already (convolution planes).
+// error_out (optional): receives the device error word as the kernels ahead have left it.
 int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_out, int policy_size, int softmax,
                       const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
-                      cudaStream_t st);
+                      cudaStream_t st, int* error_out = nullptr);
 // value_layer: the value head's first FC (its in / part fields are filled in here)
 int launch_value_head_static(const void* tower, const HeadConvWeights& value_conv, const HeadFcLayer& value_layer,
                              const float* b1, const float* w2, float b2, int H, int B, int S, float* value_out,

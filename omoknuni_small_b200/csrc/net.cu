@@ -538,7 +538,7 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
 }
 
 int forward_device(ob200_net* n, const void* input_bt, int B, float* policy_out, float* value_out,
-                   int out_kind, cudaStream_t st, const GomokuInput* gomoku = nullptr) {
+                   int out_kind, cudaStream_t st, const GomokuInput* gomoku = nullptr, int* error_out = nullptr) {
     const ob200_net_config& c = n->cfg;
     const int S = c.board_size;
     const int F = c.filters;
@@ -563,7 +563,7 @@ int forward_device(ob200_net* n, const void* input_bt, int B, float* policy_out,
     head_fc_plan(l, nl, B, n->sm_count);
     if (int rc = launch_head_fc(l, nl, B, st)) return rc;
     if (int rc = launch_head_tails(nl == 2 ? l[0] : HeadFcLayer{}, n->bp, policy_out, c.policy_size, out_kind == OB200_OUT_PROBS,
-                                   l[nl - 1], n->b1, c.value_hidden, n->w2, n->b2, value_out, B, st)) return rc;
+                                   l[nl - 1], n->b1, c.value_hidden, n->w2, n->b2, value_out, B, st, error_out)) return rc;
     counters().evals.fetch_add((uint64_t)B, std::memory_order_relaxed);
     counters().batches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;
@@ -639,6 +639,27 @@ int wait_slot(ob200_net* n, int si) {
     return rc;
 }
 
+// A batch whose results are at most this many bytes skips the copy engines: the board-resident tower reads the
+// histories from the page-locked block (every board's 34 bytes once), the last kernel writes the results there and the
+// device's error word beside them, and nothing hops between streams.  One board through the host: 112 -> IP1 us, 250
+// boards (226 KB) 176 -> IP250 us; beyond, the writes would hold up the next batch's kernels, which the copy engine
+// does not.
+constexpr size_t kInPlaceBytes = 256 * 1024;
+// ... and whose rows the last kernel writes once (longer ones it goes over several times).
+constexpr int kInPlaceOutputs = 512;
+bool results_in_place(const ob200_net* n, int B) {
+    const size_t A = n->cfg.policy_size;
+    return n->cfg.policy_kind == OB200_POLICY_FC && A <= kInPlaceOutputs && (size_t)B * (A + 1) * sizeof(float) <= kInPlaceBytes;
+}
+int forward_in_place(ob200_net* n, int si, const void* input_bt, int B, float* policy_out, float* value_out, int out_kind,
+                     const GomokuInput* gomoku) {
+    ob200_net::Slot& sl = n->slot[si];
+    sl.B = B; sl.user_policy = policy_out; sl.user_value = value_out; sl.direct = false;
+    if (int rc = forward_device(n, input_bt, B, sl.h_policy, sl.h_value, out_kind, n->stream, gomoku, sl.h_err)) return rc;
+    OB200_CUDA_OK(cudaEventRecord(sl.done, n->stream));
+    return OB200_OK;
+}
+
 // Gomoku histories -> staging -> device -> encoder -> forward -> results on their way back.  Handle mutex held.
 int enqueue_gomoku(ob200_net* n, int si, const int16_t* history, const uint8_t* n_hist, const uint8_t* to_move, int32_t B,
                    float* policy_out, float* value_out, int32_t out_kind) {
@@ -649,6 +670,10 @@ int enqueue_gomoku(ob200_net* n, int si, const int16_t* history, const uint8_t* 
     std::memcpy(h8, history, hist_bytes);
     std::memcpy(h8 + hist_bytes, n_hist, (size_t)B);
     std::memcpy(h8 + hist_bytes + B, to_move, (size_t)B);
+    if (n->resident && results_in_place(n, B)) {
+        const GomokuInput g{sl.h_hist, h8 + hist_bytes, h8 + hist_bytes + B};
+        return forward_in_place(n, si, nullptr, B, policy_out, value_out, out_kind, &g);
+    }
     // the copy goes on a stream of its own, so that it runs while the batch ahead still computes; the slot's device
     // block is free: its previous batch was waited for before the slot was handed out again
     OB200_CUDA_OK(cudaMemcpyAsync(d8, h8, hist_bytes + 2 * (size_t)B, cudaMemcpyHostToDevice, n->in_stream));
@@ -699,8 +724,12 @@ int ob200_net_infer_planes(ob200_net* n, const float* planes, int32_t B, int32_t
         cudaEventRecord(n->planes_copied, n->stream) != cudaSuccess)
         rc = set_error(OB200_ERR_CUDA, "ob200_net_infer_planes: copying the planes to the device failed");
     step(rc ? rc : launch_planes_to_board_tensor(n->d_planes, B, used, c.board_size, n->cin_pad, n->act_in, n->stream, c.tower_dtype));
-    step(rc ? rc : forward_device(n, n->act_in, B, n->slot[si].d_policy, n->slot[si].d_value, out_kind, n->stream));
-    step(rc ? rc : enqueue_results(n, si, B, policy_out, value_out));
+    if (results_in_place(n, B)) {
+        step(rc ? rc : forward_in_place(n, si, n->act_in, B, policy_out, value_out, out_kind, nullptr));
+    } else {
+        step(rc ? rc : forward_device(n, n->act_in, B, n->slot[si].d_policy, n->slot[si].d_value, out_kind, n->stream));
+        step(rc ? rc : enqueue_results(n, si, B, policy_out, value_out));
+    }
     lk.unlock();
     if (rc) { release_slot(n, si); return rc; }
     return wait_slot(n, si);
