@@ -40,6 +40,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return false;
 }
 
+// The same for a whole warp: every lane waits, and the answer is the warp's.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    for (uint32_t i = 0; i < kSpinLimit; ++i) {
+        if (__all_sync(0xFFFFFFFFu, mbar_test(bar, parity))) return true;
+        if ((i & 255) == 255 && __any_sync(0xFFFFFFFFu, *abort_flag)) return false;
+    }
+    return false;
+}
+// 1 in one lane of the (converged) warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -91,6 +106,19 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// The same, issued by the lane(s) with `on` set in a warp that runs the issue loop as a whole.
+__device__ __forceinline__ void umma_if(uint32_t on, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n.reg .b64 da, db;\n"
+        "mov.b64 da, {%1, %3};\nmov.b64 db, {%2, %3};\n"
+        "setp.ne.b32 p, %5, 0;\nsetp.ne.b32 q, %6, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t on, uint32_t bar) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar), "r"(on) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile(
