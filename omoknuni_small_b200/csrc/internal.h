@@ -63,6 +63,15 @@ int conv_wide_pack(const float* w, const float* scale, int cout, int cin_real, i
 int launch_conv_wide_maps(const BoardTensorMap& in_map, const BoardTensorMap& out_map, const BoardTensorMap* res_map,
                           const void* packed_w, const float* bias, int B, int S, int cin, int cout, int taps, int relu,
                           cudaStream_t st, float* out_f32 = nullptr, int dtype = 0);
+// The same layers on 8x8 boards over the cells alone (tower_board8.cu).  A tensor of B boards as 4-D maps (channel, x, y,
+// board); a box is 64 channels of one board row of 2 (m[0]) or 4 (m[1]) boards, what lies outside the boards reads as
+// zero.  Padding positions of the output are left as they are (zero in a handle's tensors).
+struct BoardRowMaps { BoardTensorMap m[2]; };
+int make_board_row_maps(const void* base, int S, int B, int channels, BoardRowMaps* out);
+bool conv_board8_covers(int S, int cin, int cout);
+void conv_board8_pack(const float* w, const float* scale, int cout, int cin_real, int cin, void* packed_out, int dtype);
+int launch_conv_board8(const BoardRowMaps& in, const BoardRowMaps& out, const BoardRowMaps* res, const void* packed_w, const float* bias,
+                       int B, int cin, int cout, int relu, cudaStream_t st, int dtype);
 
 // C: channels of the tower board tensor (a multiple of 64).
 // hp [B][hp_pitch], hv [B][hv_pitch]: a board's policy / value head channels, flattened as c * S*S + y * S + x

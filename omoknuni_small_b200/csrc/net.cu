@@ -19,6 +19,8 @@ struct ob200_net {
     ob200_net_config cfg{};
     int cin_pad = 64;               // channels of the input board tensor (input_channels rounded up to 64)
     bool wide = false;              // filters 128 / 256: the streamed-weight kernel; 64: the resident-weight kernel
+    bool board8 = false;            // wide, 8x8 boards: the kernel over the cells alone
+    ob200::BoardRowMaps in_rows{}, act_rows[3]{};
     int box_in = 0;                 // rows of a load box of the tower kernel in use
     long long rows = 0;             // positions per board tensor (sized for max_batch)
     ob200::BoardTensorMap in_map_load{}, act_load[3]{}, act_store[3]{};
@@ -139,7 +141,8 @@ int add_conv(ob200_net* n, const std::string& conv, const std::string& bn, int c
     std::vector<float> scale, shift;
     if (int rc = bn_fold(n, bn, F, scale, shift)) return rc;
     std::vector<uint16_t> packed((size_t)9 * cin * F);
-    if (int rc = ob200_pack_conv3x3_weights_dt(w->data(), scale.data(), F, cin_real, cin, n->cfg.tower_dtype, packed.data())) return rc;
+    if (n->board8) conv_board8_pack(w->data(), scale.data(), F, cin_real, cin, packed.data(), n->cfg.tower_dtype);
+    else if (int rc = ob200_pack_conv3x3_weights_dt(w->data(), scale.data(), F, cin_real, cin, n->cfg.tower_dtype, packed.data())) return rc;
     uint16_t* dw = nullptr; float* db = nullptr;
     if (int rc = upload(n, &dw, packed)) return rc;
     if (int rc = upload(n, &db, shift)) return rc;
@@ -259,6 +262,7 @@ int ob200_net_create(const ob200_net_config* cfg, ob200_net** out) {
     n->cfg = *cfg;
     n->cin_pad = (cfg->input_channels + 63) / 64 * 64;
     n->wide = cfg->filters != 64;
+    n->board8 = n->wide && conv_board8_covers(cfg->board_size, n->cin_pad, cfg->filters);
     n->box_in = n->wide ? conv_wide_box_rows() : 128 + 2 * conv_halo_rows(cfg->board_size);
     n->rows = board_geom(cfg->board_size, cfg->max_batch).PT;
     *out = n;
@@ -364,11 +368,15 @@ int ob200_net_finalize(ob200_net* n) {
     if (int rc = dev_alloc(n, &p8, (size_t)n->rows * n->cin_pad * 2, true)) return rc;
     n->act_in = p8;
     if (int rc = make_board_tensor_map(p8, n->rows, n->box_in, &n->in_map_load, n->cin_pad)) return rc;
+    if (n->board8)
+        if (int rc = make_board_row_maps(p8, c.board_size, c.max_batch, n->cin_pad, &n->in_rows)) return rc;
     for (int i = 0; i < 3; ++i) {
         if (int rc = dev_alloc(n, &p8, (size_t)n->rows * F * 2, true)) return rc;
         n->act[i] = p8;
         if (int rc = make_board_tensor_map(p8, n->rows, n->box_in, &n->act_load[i], F)) return rc;
         if (int rc = make_board_tensor_map(p8, n->rows, box_store, &n->act_store[i], F)) return rc;
+        if (n->board8)
+            if (int rc = make_board_row_maps(p8, c.board_size, c.max_batch, F, &n->act_rows[i])) return rc;
     }
     if (!n->wide && tower_fused_smem_bytes(c.board_size, 1 + 2 * c.blocks) != 0) {
         // one cooperative launch for the whole tower: layer descriptors with the buffer rotation of
@@ -498,6 +506,22 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
     if (!done && gomoku)       // the other tower paths read an input tensor: encode into the handle's own
         if (int rc = launch_encode_gomoku(gomoku->hist, gomoku->nh, gomoku->tm, B, S, c.input_channels, n->cin_pad, n->act_in, st,
                                           c.tower_dtype)) return rc;
+    if (n->board8) {
+        BoardRowMaps rows;
+        if (!own_input)
+            if (int rc = make_board_row_maps(input_bt, S, B, n->cin_pad, &rows)) return rc;
+        auto conv = [&](const BoardRowMaps& in, int cin, int out, const BoardRowMaps* res, int layer) {
+            return launch_conv_board8(in, n->act_rows[out], res, n->conv_w[layer], n->conv_b[layer], B, cin, F, 1, st, c.tower_dtype);
+        };
+        if (int rc = conv(own_input ? n->in_rows : rows, n->cin_pad, x, nullptr, 0)) return rc;
+        for (int i = 0; i < c.blocks; ++i) {
+            if (int rc = conv(n->act_rows[x], F, y, nullptr, 1 + 2 * i)) return rc;
+            if (int rc = conv(n->act_rows[y], F, z, &n->act_rows[x], 2 + 2 * i)) return rc;
+            std::swap(x, z);
+        }
+        n->tower_path = 0;
+        done = true;
+    }
     BoardTensorMap conv_map;
     if (!done && !own_input)
         if (int rc = input_map(n, input_bt, B, n->box_in, &conv_map)) return rc;
@@ -641,8 +665,8 @@ int wait_slot(ob200_net* n, int si) {
 
 // A batch whose results are at most this many bytes skips the copy engines: the board-resident tower reads the
 // histories from the page-locked block (every board's 34 bytes once), the last kernel writes the results there and the
-// device's error word beside them, and nothing hops between streams.  One board through the host: 112 -> IP1 us, 250
-// boards (226 KB) 176 -> IP250 us; beyond, the writes would hold up the next batch's kernels, which the copy engine
+// device's error word beside them, and nothing hops between streams.  One board through the host: 112 -> 97 us, 250
+// boards (226 KB) 176 -> 167 us; beyond, the writes would hold up the next batch's kernels, which the copy engine
 // does not.
 constexpr size_t kInPlaceBytes = 256 * 1024;
 // ... and whose rows the last kernel writes once (longer ones it goes over several times).

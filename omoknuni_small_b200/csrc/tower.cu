@@ -356,6 +356,26 @@ int make_board_plane_maps(const void* base, int S, int B, BoardPlaneMaps* out) {
     return OB200_OK;
 }
 
+int make_board_row_maps(const void* base, int S, int B, int channels, BoardRowMaps* out) {
+    const EncodeFn encode = tensor_map_encoder();
+    if (!encode) return set_error(OB200_ERR_CUDA, "cannot resolve cuTensorMapEncodeTiled from the driver");
+    if (((uintptr_t)base & 15) || S < 1 || S + 1 > 256 || B < 1 || channels < kC || channels % kC)
+        return set_error(OB200_ERR_INVALID, "board row map: base must be 16-byte aligned, channels a multiple of 64");
+    const cuuint64_t cell = (cuuint64_t)channels * 2, GP = S + 1;
+    for (int i = 0; i < 2; ++i) {
+        const cuuint64_t dims[4] = {(cuuint64_t)channels, (cuuint64_t)S, (cuuint64_t)S, (cuuint64_t)B};
+        const cuuint64_t strides[3] = {cell, GP * cell, GP * GP * cell};
+        const cuuint32_t box[4] = {(cuuint32_t)kC, (cuuint32_t)S, 1, (cuuint32_t)(i ? 4 : 2)};
+        const cuuint32_t estr[4] = {1, 1, 1, 1};
+        uint8_t* at = static_cast<uint8_t*>(const_cast<void*>(base)) + (size_t)OB200_GUARD * cell;
+        const CUresult r = encode(reinterpret_cast<CUtensorMap*>(&out->m[i]), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, at, dims, strides, box,
+                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return set_error(OB200_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+    }
+    return OB200_OK;
+}
+
 int conv_halo_rows(int S) { return S + 2; }   // |dy*(S+1)+dx| <= S+2 rows before / after a tile
 
 int launch_conv3x3_maps(const BoardTensorMap& in_map, const BoardTensorMap& out_map, const BoardTensorMap* res_map,

@@ -40,3 +40,51 @@ def test_wide_tiles_exact(lib, B, S, cin, cout, residual):
     assert capi.device_error_code() == 0
     got, pad_zero = capi.board_tensor_to_planes(out.cpu().numpy().view(np.uint16), S, B, cout)
     assert np.abs(want).max() <= 256 and np.array_equal(got, want) and pad_zero
+
+
+@pytest.mark.parametrize("F,cin,B,dtype", [
+    (128, 17, 1, 0), (128, 100, 2, 1), (128, 17, 3, 0),    # 1 and 2 input slices; half a unit, a unit, a unit and a half
+    (256, 119, 1, 0), (256, 200, 5, 1),                     # 2 and 4 slices
+    (256, 119, 74, 1), (256, 119, 75, 0),                   # the last batch of two-board units on 148 SMs, the first of four
+    (128, 17, 148, 0), (128, 17, 149, 1),
+    (256, 20, 151, 0), (256, 20, 301, 1),                   # CTAs of one and two units; of two and three, the last a quarter full
+])
+def test_board8_tower_exact(lib, F, cin, B, dtype):
+    """Towers on 8x8 boards: stem and one block, rounded to 16 bits after every layer, in exact integer arithmetic."""
+    import torch
+    import torch.nn.functional as tf
+    from omoknuni_small_b200 import capi, synth
+    rng = np.random.default_rng(F + B)
+    w = synth.make_weights(synth.net_tensor_shapes(8, cin, F, 1, 65, 2, 1), seed=1, init="torch_default", bn="identity")
+    x, w["input_conv.weight"], w["input_bn.bias"], _ = integer_layer(rng, B, 8, cin, F)
+    _, w["res_blocks.0.conv1.weight"], w["res_blocks.0.bn1.bias"], _ = integer_layer(rng, 1, 8, F, F)
+    _, w["res_blocks.0.conv2.weight"], w["res_blocks.0.bn2.bias"], _ = integer_layer(rng, 1, 8, F, F)
+    net = capi.Net(cin, 8, 1, F, 65, 2, 1, 256, B + 2, tower_dtype=dtype).load(w)
+    stored = torch.float16 if dtype else torch.bfloat16
+
+    def layer(h, conv, bn, res=0.0):
+        h = tf.conv2d(h, torch.from_numpy(w[conv]), padding=1) + torch.from_numpy(w[bn])[None, :, None, None] + res
+        assert float(h.abs().max()) < 2 ** 15
+        return h.clamp(min=0).to(stored).float()
+
+    h0 = layer(torch.from_numpy(x), "input_conv.weight", "input_bn.bias")
+    want = layer(layer(h0, "res_blocks.0.conv1.weight", "res_blocks.0.bn1.bias"), "res_blocks.0.conv2.weight", "res_blocks.0.bn2.bias", h0).numpy()
+    n16 = int(capi.lib().ob200_board_tensor_bytes(8, B, F)) // 2
+
+    class Out:
+        __cuda_array_interface__ = None
+
+    for own_input in (False, True):          # a caller's input tensor, then the handle's own
+        if own_input:
+            net.infer_planes(x)
+        else:
+            bt = torch.from_numpy(capi.planes_to_board_tensor_host(x, net.input_tensor_channels(), dtype).view(np.int16)).cuda()
+            net.tower_device(bt, B)
+        torch.cuda.synchronize()
+        Out.__cuda_array_interface__ = dict(data=(net.tower_output_ptr(), False), shape=(n16,), typestr="<i2", version=3)
+        tower = torch.as_tensor(Out(), device="cuda").cpu().numpy().view(np.uint16)
+        tower = tower.copy()
+        tower[(capi.GUARD + B * 81) * F:] = 0          # beyond the batch's boards lie the handle's other boards
+        got, pad_zero = capi.board_tensor_to_planes(tower, 8, B, F, dtype)
+        assert np.array_equal(got, want) and pad_zero, (own_input, np.abs(got - want).max())
+    assert capi.device_error_code() == 0 and np.abs(want).max() > 0
