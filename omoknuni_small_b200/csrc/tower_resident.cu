@@ -18,9 +18,9 @@
 // summed tap by tap in the order of the one-layer kernels, so the results are theirs bit for bit.
 // Smaller boards share a tile (two 10x10, four 7x7 ones) when there are more boards than SMs.
 //
-//   * Two tiles are in flight per CTA, each with its own MMA-issuing thread: while one tile's accumulators are drained
+//   * Two tiles are in flight per CTA, each with its own MMA-issuing warp: while one tile's accumulators are drained
 //     and written back as the next layer's input, the tensor cores run the other (it runs two thirds of a layer
-//     behind).  MMAs of one tile stay in one thread, so their order does not depend on the interleaving.
+//     behind).  MMAs of one tile stay in one warp, so their order does not depend on the interleaving.
 //   * Sixteen epilogue warps: a warp owns one TMEM lane quadrant, one parity and 32 of the 64 channels.
 //   * Weights stream from L2 through a one-layer ring of three 24 KB blocks (three taps of one dy each): a block is
 //     handed back by a tcgen05.commit of every issuer, and the loader refills it with the next layer's when all have
@@ -39,6 +39,9 @@
 // GEMM row), 4,600 for a lone one (5,450).  From some hundred boards on the GPU runs at its 1,000 W limit (1.75 GHz in
 // these kernels), which takes part of that back: 4,096 boards 1,290 -> 1,230 us cold, 1,390 -> 1,320 us sustained.
 // 1 board 70 -> 58 us; the 32 / 32-channel heads' convolutions, 31-47 us as a launch of their own before, 2 us.
+// With the issuing warp in its loop as a whole (a lone lane moves every MMA's descriptors to uniform registers), an
+// evaluation on the device, 2 / 1-channel heads: 250 boards 99 -> 83 us, 1,024 boards 333 -> 280, 4,096 boards 1,218 ->
+// 1,031 on a cool GPU, one board 65.6 -> 63.6.
 #include "internal.h"
 #include "sm100_ptx.cuh"
 #include "head_conv.cuh"
@@ -221,8 +224,11 @@ conv_tower_resident_kernel(const __grid_constant__ CUtensorMap in_even, const __
         // ---------------- MMA issuers: warp 16 + bd for tile bd of the round ----------------
         // Tile 1 runs two thirds of a layer behind tile 0 (its issuer starts a layer when tile 0's has issued two of the
         // three weight blocks), so that one tile's MMAs cover the other's epilogue.
-        const int bd = warp - kEpiWarps;
-        if (lane == 0 && (PAIR || bd == 0)) {
+        // The warp runs the loop as a whole and one lane issues: with loop state the compiler knows to be the warp's, the
+        // descriptors stay in uniform registers.
+        const int bd = __shfl_sync(0xFFFFFFFFu, warp, 0) - kEpiWarps;
+        if (PAIR || bd == 0) {
+            const uint32_t lead = elect_one();
             constexpr uint32_t kIdesc64 = make_idesc(F16, kTileM, kC), kIdesc128 = make_idesc(F16, kTileM, 2 * kC);
             constexpr uint32_t kRow = kRowBytes >> 4, kTap = kTapBytes >> 4;
             const uint32_t w_lo = desc_lo(smem_u32(w_s));
@@ -236,14 +242,14 @@ conv_tower_resident_kernel(const __grid_constant__ CUtensorMap in_even, const __
                 if (n >= n_my) break;                   // a single tile in the last round: tile 1's issuer is done
                 const uint32_t even = act_lo + (plane_off(n, 0) >> 4), odd = act_lo + (plane_off(n, 1) >> 4);
                 for (int l = 0; l < LL; ++l) {
-                    if (l == 0 && !mbar_wait(in_full(bd), (uint32_t)round & 1u, abort_flag)) { ok = false; break; }
+                    if (l == 0 && !mbar_wait_warp(in_full(bd), (uint32_t)round & 1u, abort_flag)) { ok = false; break; }
                     if (round + l > 0) {
-                        if (!mbar_wait(act_ready(bd), ready_cnt & 1u, abort_flag)) { ok = false; break; }
+                        if (!mbar_wait_warp(act_ready(bd), ready_cnt & 1u, abort_flag)) { ok = false; break; }
                         ++ready_cnt;
                     }
                     if (l == L) {
                         // the heads' 1x1 convolutions: [W0 | W1] and, on top of W1's sums, W2
-                        if (!mbar_wait(w_full(0), uses[0] & 1u, abort_flag)) { ok = false; break; }
+                        if (!mbar_wait_warp(w_full(0), uses[0] & 1u, abort_flag)) { ok = false; break; }
                         ++uses[0];
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const int hr = p.head_rows;
@@ -253,15 +259,15 @@ conv_tower_resident_kernel(const __grid_constant__ CUtensorMap in_even, const __
 #pragma unroll
                             for (int ks = 0; ks < kC / 16; ++ks) {
                                 const uint32_t a = (par ? odd : even) + ks * 2, dh = d + (uint32_t)(par * 2 * hr);
-                                umma(dh, a, w_lo + ks * 2, id2, ks ? 1u : 0u);
-                                umma(dh + (uint32_t)hr, a, w_lo + (uint32_t)(2 * hr) * kRow + ks * 2, id1, 1u);
+                                umma_if(lead, dh, a, w_lo + ks * 2, id2, ks ? 1u : 0u);
+                                umma_if(lead, dh + (uint32_t)hr, a, w_lo + (uint32_t)(2 * hr) * kRow + ks * 2, id1, 1u);
                             }
-                        umma_commit(w_empty(0));
-                        umma_commit(acc_full(bd));
+                        umma_commit_if(lead, w_empty(0));
+                        umma_commit_if(lead, acc_full(bd));
                         continue;
                     }
                     if (bd == 1) {
-                        if (!mbar_wait(stagger, stagger_cnt & 1u, abort_flag)) { ok = false; break; }
+                        if (!mbar_wait_warp(stagger, stagger_cnt & 1u, abort_flag)) { ok = false; break; }
                         ++stagger_cnt;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -269,31 +275,31 @@ conv_tower_resident_kernel(const __grid_constant__ CUtensorMap in_even, const __
                     for (int dy = 0; dy < 3; ++dy) {
                         // weights are waited for and handed back three taps at a time (a wait costs the issuing
                         // thread about 50 cycles, a commit 25)
-                        if (!mbar_wait(w_full(dy), uses[dy] & 1u, abort_flag)) { ok = false; break; }
+                        if (!mbar_wait_warp(w_full(dy), uses[dy] & 1u, abort_flag)) { ok = false; break; }
                         ++uses[dy];
                         const uint32_t e = even + (uint32_t)dy * dy_step - dy_step, o = odd + (uint32_t)dy * dy_step - dy_step;
                         const uint32_t w = w_lo + (uint32_t)(dy * 3) * kTap;
 #pragma unroll
-                        for (int ks = 0; ks < kC / 16; ++ks) umma(d_even, o - kRow + ks * 2, w + ks * 2, kIdesc64, (dy | ks) ? 1u : 0u);
+                        for (int ks = 0; ks < kC / 16; ++ks) umma_if(lead, d_even, o - kRow + ks * 2, w + ks * 2, kIdesc64, (dy | ks) ? 1u : 0u);
 #pragma unroll
                         for (int ks = 0; ks < kC / 16; ++ks) {
                             if (dy == 0 && ks == 0) {          // the odd cells' sums start here, the even cells' have begun
-                                umma(d_odd, e, w, kIdesc64, 0u);
-                                umma(d_even, e, w + kTap, kIdesc64, 1u);
-                            } else umma(d, e + ks * 2, w + ks * 2, kIdesc128, 1u);
+                                umma_if(lead, d_odd, e, w, kIdesc64, 0u);
+                                umma_if(lead, d_even, e, w + kTap, kIdesc64, 1u);
+                            } else umma_if(lead, d, e + ks * 2, w + ks * 2, kIdesc128, 1u);
                         }
 #pragma unroll
-                        for (int ks = 0; ks < kC / 16; ++ks) umma(d, o + ks * 2, w + kTap + ks * 2, kIdesc128, 1u);
+                        for (int ks = 0; ks < kC / 16; ++ks) umma_if(lead, d, o + ks * 2, w + kTap + ks * 2, kIdesc128, 1u);
 #pragma unroll
-                        for (int ks = 0; ks < kC / 16; ++ks) umma(d_odd, e + kRow + ks * 2, w + 2 * kTap + ks * 2, kIdesc64, 1u);
-                        umma_commit(w_empty(dy));
-                        if (PAIR && dy == 1 && bd == 0) mbar_arrive(stagger);
+                        for (int ks = 0; ks < kC / 16; ++ks) umma_if(lead, d_odd, e + kRow + ks * 2, w + 2 * kTap + ks * 2, kIdesc64, 1u);
+                        umma_commit_if(lead, w_empty(dy));
+                        if (PAIR && dy == 1 && bd == 0 && lead) mbar_arrive(stagger);
                     }
                     if (!ok) break;
-                    umma_commit(acc_full(bd));
+                    umma_commit_if(lead, acc_full(bd));
                 }
             }
-            if (!ok) { *abort_flag = 1; atomicExch(p.error, 2); }
+            if (!ok && lead) { *abort_flag = 1; atomicExch(p.error, 2); }
         }
     } else {
         // ---------------- epilogue: TMEM -> registers -> the next layer's input rows, in place ----------------
