@@ -149,12 +149,12 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(w_bar, 0, abort_flag);
-            if (!ok) { *abort_flag = 1; atomicExch(p.error, 2); }
-            // Everything that does not change from tile to tile is prepared once: the issuing
-            // thread is a single warp lane, so each MMA must cost it a handful of integer
-            // instructions, not a descriptor rebuild.
+        {
+            const uint32_t lead = elect_one();       // the warp runs the loop as a whole, one lane issues
+            bool ok = mbar_wait_warp(w_bar, 0, abort_flag);
+            if (!ok && lead) { *abort_flag = 1; atomicExch(p.error, 2); }
+            // Everything that does not change from tile to tile is prepared once: each MMA must
+            // cost the issuing warp a handful of integer instructions, not a descriptor rebuild.
             const uint32_t w_lo = desc_lo(smem_u32(w_s));
             int tap_off[9];
 #pragma unroll
@@ -164,8 +164,9 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant
             int s = 0, a = 0;
             uint32_t ph = 0, pa = 0;
             for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
-                if (!mbar_wait(accempty_bar(a), pa ^ 1u, abort_flag) || !mbar_wait(full_bar(s), ph, abort_flag)) {
-                    *abort_flag = 1; atomicExch(p.error, 2); break;
+                if (!mbar_wait_warp(accempty_bar(a), pa ^ 1u, abort_flag) || !mbar_wait_warp(full_bar(s), ph, abort_flag)) {
+                    if (lead) { *abort_flag = 1; atomicExch(p.error, 2); }
+                    break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a_lo = a_base + (uint32_t)(s * (kStageBytes >> 4));
@@ -174,11 +175,11 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant
                 for (int tap = 0; tap < 9; ++tap) {
 #pragma unroll
                     for (int ks = 0; ks < kC / 16; ++ks)
-                        umma(d_tmem, a_lo + (uint32_t)(tap_off[tap] + ks * 2),
+                        umma_if(lead, d_tmem, a_lo + (uint32_t)(tap_off[tap] + ks * 2),
                              w_lo + (uint32_t)(tap * (kC * kRowBytes >> 4) + ks * 2), kIdesc, (tap | ks) ? 1u : 0u);
                 }
-                umma_commit(empty_bar(s));      // smem stage free once these MMAs have read it
-                umma_commit(accfull_bar(a));    // accumulator ready for the epilogue
+                umma_commit_if(lead, empty_bar(s));      // smem stage free once these MMAs have read it
+                umma_commit_if(lead, accfull_bar(a));    // accumulator ready for the epilogue
                 if (++s == kStages) { s = 0; ph ^= 1u; }
                 if (++a == kAccStages) { a = 0; pa ^= 1u; }
             }
