@@ -37,7 +37,7 @@ struct ob200_net {
     int tower_path = -1;            // path of the last forward: 0 per layer, 1 cooperative launch, 2 board-resident
     // the fused tower (64 filters): per-layer descriptors and tile flags on the device
     void* fused_layers = nullptr; int *fused_flags = nullptr, *fused_done = nullptr; int fused_pitch = 0, fused_epoch = 0, fused_final = 0;
-    bool fused = false, fused_forced = false;   // forced: OB200_TOWER_FUSED=2 (tests: every batch size)
+    bool fused = false;                         // OB200_TOWER_FUSED=2
     // the board-resident tower (64 filters, boards up to 15x15): layer descriptors, whole-board boxes
     void** resident_layers = nullptr; bool resident = false;
     std::vector<float> resident_bias;                // [1 + 2 * blocks][64]
@@ -400,8 +400,7 @@ int ob200_net_finalize(ob200_net* n) {
         n->fused_pitch = (int)(board_geom(c.board_size, c.max_batch).Ppad / 128);
         if (int rc = dev_alloc(n, &n->fused_flags, (size_t)L * n->fused_pitch, true)) return rc;
         if (int rc = dev_alloc(n, &n->fused_done, (size_t)L, true)) return rc;
-        n->fused = !(env && env[0] == '0');
-        n->fused_forced = env && env[0] == '2';
+        n->fused = env && env[0] == '2';
     }
     if (!n->wide && n->cin_pad == 64 && tower_resident_covers(c.board_size, 1 + 2 * c.blocks)) {
         // boards stay in shared memory through all the layers: one ordinary launch
@@ -526,20 +525,14 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
     if (!done && !own_input)
         if (int rc = input_map(n, input_bt, B, n->box_in, &conv_map)) return rc;
     const BoardTensorMap& in_map = own_input ? n->in_map_load : conv_map;
-    // The fused tower pays off in a window of batch sizes (measured, 15x15: 4.5 % faster at 1,024 boards,
-    // equal at 512, 45 % slower at 64, 19 % slower at 4,096).  Below about 8 tiles per CTA and layer the
-    // hand-over of tiles through flags in global memory (store complete -> flag -> poll, about 3 us per
-    // layer on the critical path) costs more than a kernel boundary; and it keeps two activation tiles
-    // in flight per CTA, which covers L2 latency but not DRAM latency, so the three rotating
-    // activation tensors must stay resident in L2 (40 MB each at most; 15x15 boards: 1,220 per batch).
-    const BoardGeom bg = board_geom(S, B);
-    const bool l2_resident = (size_t)bg.PT * 128 <= ((size_t)40 << 20);
-    const bool enough_tiles = bg.Ppad / 128 >= 8LL * n->sm_count;
+    // The one-launch tower runs only when asked for (OB200_TOWER_FUSED=2): handing tiles over through flags in global
+    // memory (store complete -> flag -> poll, about 3 us a layer) now costs more than kernel boundaries at every size.
+    // 19x19, 21 layers, a launch per layer against one launch: 400 boards 276 / 308 us, 550 350 / 370, 780 503 / 541.
     // The tile flags carry a per-launch epoch kept on the host: a launch replayed from a captured
     // graph would see its own earlier flags, so a capturing stream gets the per-layer kernels.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) { cudaGetLastError(); capturing = cudaStreamCaptureStatusNone; }
-    if (!done && n->fused && capturing == cudaStreamCaptureStatusNone && (n->fused_forced || (l2_resident && enough_tiles))) {
+    if (!done && n->fused && capturing == cudaStreamCaptureStatusNone) {
         if (++n->fused_epoch == 0) ++n->fused_epoch;   // flags start at zero: epoch 0 is never used
         const int rc = launch_conv_tower(in_map, n->fused_layers, 1 + 2 * c.blocks, n->fused_flags, n->fused_pitch,
                                          n->fused_done, n->fused_epoch, B, S, st, c.tower_dtype);
