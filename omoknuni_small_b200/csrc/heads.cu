@@ -271,15 +271,20 @@ void head_conv_pack(const float* w, int hc, int C, int dtype, void* packed_out, 
             for (int t = 0; t < 3; ++t) {
                 uint16_t u;
                 float f;
+                uint32_t bits;
+                std::memcpy(&bits, &v, 4);
                 if (dtype == OB200_DTYPE_F16) {
-                    u = f32_to_f16_rne_sat(v);
+                    // an infinite weight stays one
+                    u = std::isinf(v) ? (uint16_t)(((bits >> 16) & 0x8000u) | 0x7C00u) : f32_to_f16_rne_sat(v);
                     f = __half2float(*reinterpret_cast<const __half*>(&u));
                 } else {
                     u = f32_to_bf16_rne(v);
+                    if ((u & 0x7FFFu) == 0x7F80u) u = (uint16_t)(bits >> 16);      // a finite one does not become one
                     const uint32_t b = (uint32_t)u << 16;
                     std::memcpy(&f, &b, 4);
                 }
                 std::memcpy(at + (size_t)t * rows * 128, &u, 2);
+                if (!std::isfinite(v)) break;                                       // no lower terms
                 v -= f;
             }
         }
