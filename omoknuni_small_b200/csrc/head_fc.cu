@@ -24,6 +24,7 @@
 // -> 221 us (that kernel took 236 us for either: eight CTAs' worth of a serial loop over 7,200 terms).
 #include "internal.h"
 #include "sm100_ptx.cuh"
+#include "head_conv.cuh"
 
 namespace ob200 {
 namespace {
@@ -160,7 +161,7 @@ head_fc_kernel(const SplitParams p) {
         const int sub = lane >> 3, kv = (lane & 7) * 4;                  // four rows a step, eight float4 a row
         float4 xs[2][4];                                                 // this stage's and the next one's
         // Loads without a condition, so that they stay in flight until their stage is split: boards beyond the batch
-        // repeat the last one (their outputs are dropped), terms beyond K repeat real ones (their weights are zero).
+        // repeat the last one (their outputs are dropped), terms beyond K repeat real ones (and are cleared below).
         const float* src_row[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) src_row[r] = L.in + (size_t)min(row0 + warp * 16 + r * 4 + sub, p.B - 1) * L.in_pitch;
@@ -207,17 +208,20 @@ head_fc_kernel(const SplitParams p) {
             if (!__all_sync(0xffffffffu, good)) { ok = false; return; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t t = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 2 * kN + half * 64);
-            const bool opens = c == chunk0 || c % kHeadFcGroup == 0;
+            if (c == chunk0 || c % kHeadFcGroup == 0) {
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                uint32_t r[16], small[16];
-                tmem_ld16(t + h * 16, r);
-                tmem_ld16(t + kN + h * 16, small);
+                for (int j = 0; j < 64; ++j) group[j] = -0.0f;          // -0 + v is v for every v
+            }
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+                uint32_t r[8], small[8];
+                tmem_ld8(t + h * 8, r);
+                tmem_ld8(t + kN + h * 8, small);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float v = __fadd_rn(__uint_as_float(r[j]), __uint_as_float(small[j]));
-                    group[h * 16 + j] = opens ? v : __fadd_rn(group[h * 16 + j], v);
+                for (int j = 0; j < 8; ++j) {
+                    const float v = join_terms(__uint_as_float(r[j]), __uint_as_float(small[j]));
+                    group[h * 8 + j] = __fadd_rn(group[h * 8 + j], v);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -233,6 +237,17 @@ head_fc_kernel(const SplitParams p) {
             const bool good = mbar_wait(empty(s), ((uint32_t)(i / kStages) & 1u) ^ 1u, abort_flag);
             if (!__all_sync(0xffffffffu, good)) { ok = false; return; }
             uint8_t* dst = smem + s * kStageBytes;
+            // terms beyond K have weights of zero, but an infinity repeated there would make NaN of them
+            const int left = L.K - ((kb0 + i) * kStageK + kv);
+            if (left < 4) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if (left < 1) x[r].x = 0.0f;
+                    if (left < 2) x[r].y = 0.0f;
+                    if (left < 3) x[r].z = 0.0f;
+                    x[r].w = 0.0f;
+                }
+            }
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int row = warp * 16 + r * 4 + sub;
@@ -275,6 +290,15 @@ size_t head_fc_packed_bytes(int K, int N) {
     return (size_t)((N + kN - 1) / kN) * ((K + kStageK - 1) / kStageK) * kOperandBytes;
 }
 
+// The three terms of a weight, as split2 makes them, but a finite one has finite terms up to fp32's largest number.
+__device__ __forceinline__ void split_weight(float x, uint16_t (&t)[3]) {
+    for (int s = 0; s < 3; ++s) {
+        float lead = __bfloat162float(__float2bfloat16_rn(x));
+        if (fabsf(lead) == INFINITY && fabsf(x) < INFINITY) lead = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+        t[s] = (uint16_t)(__float_as_uint(lead) >> 16);
+        x = __fsub_rn(x, lead);
+    }
+}
 // w [N][K] fp32 -> blocks [output tile][32 inner terms][split term] of 128 outputs x 32 terms in bf16, 64 bytes an
 // output, 16-byte chunks permuted by the 64-byte swizzle; outputs and terms beyond N and K are zero.
 __global__ void head_fc_pack_kernel(const float* __restrict__ w, int K, int N, int k_blocks, uint8_t* __restrict__ packed) {
@@ -284,10 +308,11 @@ __global__ void head_fc_pack_kernel(const float* __restrict__ w, int K, int N, i
         const int r = i / (kStageK / 2), k = (i % (kStageK / 2)) * 2;
         const int n = tile * kN + r, gk = kb * kStageK + k;
         const float* src = w + (size_t)n * K + gk;
-        uint32_t t[3];
-        split2(n < N && gk < K ? src[0] : 0.0f, n < N && gk + 1 < K ? src[1] : 0.0f, t[0], t[1], t[2]);
+        uint16_t t0[3], t1[3];
+        split_weight(n < N && gk < K ? src[0] : 0.0f, t0);
+        split_weight(n < N && gk + 1 < K ? src[1] : 0.0f, t1);
         for (int s = 0; s < 3; ++s)
-            *reinterpret_cast<uint32_t*>(block + s * kTileBytes + r * kRowBytes + (((k >> 3) ^ ((r >> 1) & 3)) << 4) + (k & 7) * 2) = t[s];
+            *reinterpret_cast<uint32_t*>(block + s * kTileBytes + r * kRowBytes + (((k >> 3) ^ ((r >> 1) & 3)) << 4) + (k & 7) * 2) = t0[s] | (uint32_t)t1[s] << 16;
     }
 }
 int head_fc_pack(const float* w_dev, int K, int N, void* packed_dev, cudaStream_t st) {

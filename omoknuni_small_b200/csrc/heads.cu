@@ -226,7 +226,7 @@ head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __
     } else {
         const int b = (int)blockIdx.x - policy_rows;
         float s = 0.0f;
-        for (int i = threadIdx.x; i < H; i += kTailThreads) s = fmaf(fmaxf(__fadd_rn(sum_slices(val, b, B, i), b1[i]), 0.0f), w2[i], s);
+        for (int i = threadIdx.x; i < H; i += kTailThreads) s = fmaf(relu_keep_nan(__fadd_rn(sum_slices(val, b, B, i), b1[i])), w2[i], s);
         s = block_reduce(s, false, red);
         if (threadIdx.x == 0) value[b] = tanhf(s + b2);
     }

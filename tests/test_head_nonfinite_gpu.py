@@ -100,3 +100,34 @@ def test_head_convolution_with_weights_out_of_range(lib, monkeypatch, S, residen
     finite = np.isfinite(want)
     assert finite.all() == bool(np.isfinite(weight)) and not np.isfinite(logits[~finite]).any()
     assert (np.abs(logits[finite] - want[finite]) <= 2e-5 * scale[finite]).all()
+
+
+@pytest.mark.parametrize("S,resident", [(5, "1"), (8, "0"), (15, "1"), (19, "0")])
+@pytest.mark.parametrize("n_inf", [1, 2])
+def test_fully_connected_layers_of_infinities(lib, monkeypatch, S, resident, n_inf):
+    """Every logit and value is the infinity, the NaN or the number that fp32 products give; K = 75 to 1,083 terms, which
+    end inside a block of 32, the last cell infinite among others."""
+    def change(w):
+        w["policy_conv.weight"][:, :2] = np.abs(w["policy_conv.weight"][:, :2]) * np.sign(w["policy_bn.weight"])[:, None, None, None]
+        w["policy_fc.weight"][0] = np.abs(w["policy_fc.weight"][0])
+        w["policy_fc.weight"][1] = -np.abs(w["policy_fc.weight"][1])
+        w["policy_fc.weight"][2] = 0.0
+        w["policy_fc.weight"][3] = 2.0 ** -3                            # one term: the lower two of the split are zero
+    logits, value, want, scale, want_v = run(monkeypatch, S, 3, 2, n_inf, resident, change)
+    assert set(np.unique(class_of(want))) == {-1, 0, 1, 2}
+    assert np.array_equal(class_of(logits), class_of(want)) and np.array_equal(class_of(value), class_of(want_v))
+    finite = np.isfinite(want)
+    assert (np.abs(logits[finite] - want[finite]) <= 2e-5 * scale[finite]).all()
+    assert np.allclose(value[np.isfinite(want_v)], want_v[np.isfinite(want_v)], atol=1e-5)
+
+
+@pytest.mark.parametrize("weight", [np.inf, np.nan, 3.4e38, -3.4e38])
+def test_fully_connected_weights_out_of_range(lib, monkeypatch, weight):
+    def change(w):
+        w["policy_bn.weight"] *= 0.05                                   # inputs well below one
+        w["policy_bn.bias"] *= 0.05
+        w["policy_fc.weight"][7, 0] = weight
+    logits, _, want, scale, _ = run(monkeypatch, 15, 3, 2, 0, "1", change)
+    assert np.array_equal(class_of(logits), class_of(want))
+    finite = np.isfinite(want)
+    assert (np.abs(logits[finite] - want[finite]) <= 2e-5 * scale[finite]).all() and finite[:, 8:].all()
