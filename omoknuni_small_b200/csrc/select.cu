@@ -135,7 +135,10 @@ __device__ __forceinline__ int select_row(const ob200_tree_view& t, int node, fl
 //   with it; the exact pass over { s~ + kBracket*m >= T } in slot order therefore sees
 //   i* and everything that could beat or tie it.  NaN brackets compare false (never a
 //   candidate, as NaN scores are never selected) and are ignored by the maximum.
+// The bound is relative, and among subnormal numbers rounding is not: there s~ may be a few units of 2^-149 off.  Every
+// bound is therefore widened by the smallest normal number, which the larger scores do not notice.
 constexpr float kBracket = 1.9073486328125e-06f;   // 2^-19
+constexpr float kBracketMin = FLT_MIN;
 
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
@@ -300,7 +303,7 @@ puct_select_staged_kernel(ob200_tree_view t, const int32_t* __restrict__ node_id
                 bracket(nn.z, ww.z, pp.z, ll.z, explore, m & 4u, lo, hi[4 * h + 2]); lane_lo = fmaxf(lane_lo, lo);
                 bracket(nn.w, ww.w, pp.w, ll.w, explore, m & 8u, lo, hi[4 * h + 3]); lane_lo = fmaxf(lane_lo, lo);
             }
-            lane_lo = warp_max(lane_lo);
+            lane_lo = __fsub_rn(warp_max(lane_lo), kBracketMin);
             // pass 2: the slots whose bracket reaches the best lower bound.  Usually there is
             // exactly one, and with a finite bound it is the answer without any exact score.
             uint32_t cand = 0;
@@ -497,9 +500,9 @@ puct_select_segmented_kernel(ob200_tree_view t, const int32_t* __restrict__ node
         const float4* W4 = reinterpret_cast<const float4*>(st + kRowBytes);
         const float4* P4 = reinterpret_cast<const float4*>(st + 2 * kRowBytes);
         const int4* V4 = reinterpret_cast<const int4*>(st + 3 * kRowBytes);
-        // Approximate scores s~ (one MUFU reciprocal per division) with |s - s~| < kBracket * m, m = |q~| + |u~|;
-        // M = the largest m of the segment bounds every slot's error, so the segment's exact maximum is attained
-        // among the slots with s~ >= max s~ - 2 kBracket M.
+        // Approximate scores s~ (one MUFU reciprocal per division) with |s - s~| < kBracket * m, m = |q~| + |u~|
+        // (see bracket() for subnormal ones); M = the largest m of the segment bounds every slot's error, so the
+        // segment's exact maximum is attained among the slots with s~ >= max s~ - 2 kBracket M - kBracketMin.
         float sc[8];
         float lane_s = -INFINITY, lane_m = 0.0f;
         uint32_t range = 0;
@@ -527,7 +530,7 @@ puct_select_segmented_kernel(ob200_tree_view t, const int32_t* __restrict__ node
         }
         lane_s = warp_max(lane_s);
         lane_m = warp_max(lane_m);
-        float thr = fmaf(-2.0f * kBracket, lane_m, lane_s);
+        float thr = __fsub_rn(fmaf(-2.0f * kBracket, lane_m, lane_s), kBracketMin);
         thr = thr == thr ? thr : -INFINITY;       // inf - inf: no usable bound, every existing slot is a candidate
         uint32_t cand = 0;
 #pragma unroll
@@ -762,7 +765,7 @@ __device__ __forceinline__ int select_row_narrow(const ob200_tree_view& t, int n
     }
     lane_s = warp_max(lane_s);
     lane_m = warp_max(lane_m);
-    float thr = fmaf(-2.0f * kBracket, lane_m, lane_s);
+    float thr = __fsub_rn(fmaf(-2.0f * kBracket, lane_m, lane_s), kBracketMin);
     thr = thr == thr ? thr : -INFINITY;
     uint32_t cand = 0;
 #pragma unroll
