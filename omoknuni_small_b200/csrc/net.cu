@@ -656,17 +656,23 @@ int wait_slot(ob200_net* n, int si) {
     return rc;
 }
 
-// A batch whose results are at most this many bytes skips the copy engines: the board-resident tower reads the
-// histories from the page-locked block (every board's 34 bytes once), the last kernel writes the results there and the
-// device's error word beside them, and nothing hops between streams.  One board through the host: 112 -> 97 us, 250
-// boards (226 KB) 176 -> 167 us; beyond, the writes would hold up the next batch's kernels, which the copy engine
-// does not.
+// A batch whose results are at most this many bytes, with no other call in flight on the handle, skips the copy engines:
+// the board-resident tower reads the histories from the page-locked block (every board's 34 bytes once), the last kernel
+// writes the results there and the device's error word beside them, and nothing hops between streams.
+// In place / copied, a call at a time, outputs pageable: one board 101 us / 111, 64 boards 105 / 117, 256 boards (231 KB)
+// 153 / 170; page-locked, which the copy engine writes directly: 96 / 110, 105 / 113, 153 / 153, and beyond the limit 350
+// boards 216 / 205, 1,024 boards 473 / 417.
+// With another call in flight the writes hold up its kernels, which the copy engine does not.  Two calls in flight, per
+// batch: 64 boards 83 us / 75, 256 boards 123 / 108; four threads, 256 boards 150 / 109.
 constexpr size_t kInPlaceBytes = 256 * 1024;
-// ... and whose rows the last kernel writes once (longer ones it goes over several times).
+// ... and whose rows the last kernel writes once (longer ones it goes over several times: 513 outputs, 16 boards 97 us in
+// place / 103 copied, 4,096 outputs, 128 boards, 303 / 289).
 constexpr int kInPlaceOutputs = 512;
-bool results_in_place(const ob200_net* n, int B) {
+// Handle mutex held; si: the call's own slot.
+bool results_in_place(const ob200_net* n, int si, int B) {
     const size_t A = n->cfg.policy_size;
-    return n->cfg.policy_kind == OB200_POLICY_FC && A <= kInPlaceOutputs && (size_t)B * (A + 1) * sizeof(float) <= kInPlaceBytes;
+    return !n->slot[1 - si].busy && n->cfg.policy_kind == OB200_POLICY_FC && A <= kInPlaceOutputs &&
+           (size_t)B * (A + 1) * sizeof(float) <= kInPlaceBytes;
 }
 int forward_in_place(ob200_net* n, int si, const void* input_bt, int B, float* policy_out, float* value_out, int out_kind,
                      const GomokuInput* gomoku) {
@@ -687,7 +693,7 @@ int enqueue_gomoku(ob200_net* n, int si, const int16_t* history, const uint8_t* 
     std::memcpy(h8, history, hist_bytes);
     std::memcpy(h8 + hist_bytes, n_hist, (size_t)B);
     std::memcpy(h8 + hist_bytes + B, to_move, (size_t)B);
-    if (n->resident && results_in_place(n, B)) {
+    if (n->resident && results_in_place(n, si, B)) {
         const GomokuInput g{sl.h_hist, h8 + hist_bytes, h8 + hist_bytes + B};
         return forward_in_place(n, si, nullptr, B, policy_out, value_out, out_kind, &g);
     }
@@ -741,7 +747,7 @@ int ob200_net_infer_planes(ob200_net* n, const float* planes, int32_t B, int32_t
         cudaEventRecord(n->planes_copied, n->stream) != cudaSuccess)
         rc = set_error(OB200_ERR_CUDA, "ob200_net_infer_planes: copying the planes to the device failed");
     step(rc ? rc : launch_planes_to_board_tensor(n->d_planes, B, used, c.board_size, n->cin_pad, n->act_in, n->stream, c.tower_dtype));
-    if (results_in_place(n, B)) {
+    if (results_in_place(n, si, B)) {
         step(rc ? rc : forward_in_place(n, si, n->act_in, B, policy_out, value_out, out_kind, nullptr));
     } else {
         step(rc ? rc : forward_device(n, n->act_in, B, n->slot[si].d_policy, n->slot[si].d_value, out_kind, n->stream));
