@@ -48,9 +48,19 @@ int ensure_stage(ob200_tree* t, size_t bytes) {
     return OB200_OK;
 }
 
-// Selections beyond this many nodes copy their ids and results: the kernels for large launches look ids up in the
-// middle of their row pipelines, where a trip to host memory would stall them, and write results four bytes at a time.
+// Selections beyond this many nodes copy their ids and results.  In place / copied: 512 nodes of 225 slots 20.6 us / 24.5
+// (513 nodes), of 4,672 slots 28.8 / 34.7 (16 and 64 nodes: the same); 4,096 nodes of 225 slots 30 / 36, 16,384 58 / 57,
+// 65,536 164 / 135.
 constexpr int kSelectInPlace = 512;
+
+// Priors beyond this many bytes are copied, unless their rows are whole 128-byte lines: a warp's 128 bytes of a row that
+// is not straddle two lines, and the second of them crosses the bus twice.  In place / copied: 64 nodes of 225 slots
+// 21 us / 24, of 362 24 / 30; 256 of 362 43 / 41; 2,048 of 225 173 / 162, of 362 273 / 252; 64 of 4,672 101 / 112, 512
+// 750 / 760.
+constexpr size_t kPriorsInPlace = 256 * 1024;
+// Paths beyond this many bytes are copied as well.  In place / copied: 4,096 of 16 edges (0.5 MB) 109 us / 124, 16,384 of
+// 16 (2 MB) 470 / 445, 65,536 of 6 (3 MB) 1,048 / 990, of 16 1,830 / 1,716.
+constexpr size_t kPathsInPlace = 1 << 20;
 
 // Lays host arrays out in the staging block (256-byte aligned pieces).
 struct Stager {
@@ -269,8 +279,11 @@ int ob200_tree_backup(ob200_tree* t, const int32_t* paths, const int32_t* path_l
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, paths, pb); std::memcpy(t->h_stage + b, path_len, (size_t)n * 4);
     std::memcpy(t->h_stage + c, leaf_values, (size_t)n * 4);
-    if (int rc = ob200_launch_backup(&t->view, reinterpret_cast<int32_t*>(t->h_stage + a), reinterpret_cast<int32_t*>(t->h_stage + b),
-                                     reinterpret_cast<float*>(t->h_stage + c), n, max_depth, vl_value, t->stream)) return rc;
+    const bool in_place = pb <= kPathsInPlace;
+    unsigned char* stage = in_place ? t->h_stage : t->d_stage;
+    if (!in_place) OB200_CUDA_OK(cudaMemcpyAsync(stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
+    if (int rc = ob200_launch_backup(&t->view, reinterpret_cast<int32_t*>(stage + a), reinterpret_cast<int32_t*>(stage + b),
+                                     reinterpret_cast<float*>(stage + c), n, max_depth, vl_value, t->stream)) return rc;
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     return OB200_OK;
 }
@@ -285,7 +298,11 @@ int ob200_tree_set_priors(ob200_tree* t, const int32_t* node_ids, int32_t n, con
     const size_t a = s.reserve((size_t)n * 4), b = s.reserve((size_t)n * policy_size * 4);
     if (int rc = ensure_stage(t, s.used)) return rc;
     std::memcpy(t->h_stage + a, node_ids, (size_t)n * 4); std::memcpy(t->h_stage + b, policy, (size_t)n * policy_size * 4);
-    if (int rc = ob200_launch_set_priors(&t->view, reinterpret_cast<int32_t*>(t->h_stage + a), n, reinterpret_cast<float*>(t->h_stage + b),
+    const size_t row_bytes = (size_t)policy_size * 4;
+    const bool in_place = n * row_bytes <= kPriorsInPlace || row_bytes % 128 == 0;
+    unsigned char* stage = in_place ? t->h_stage : t->d_stage;
+    if (!in_place) OB200_CUDA_OK(cudaMemcpyAsync(stage, t->h_stage, s.used, cudaMemcpyHostToDevice, t->stream));
+    if (int rc = ob200_launch_set_priors(&t->view, reinterpret_cast<int32_t*>(stage + a), n, reinterpret_cast<float*>(stage + b),
                                          policy_size, nullptr, t->stream)) return rc;
     OB200_CUDA_OK(cudaStreamSynchronize(t->stream));
     return OB200_OK;
