@@ -35,7 +35,7 @@ struct ob200_net {
     void* act[3] = {nullptr, nullptr, nullptr};      // filters channels each
     const void* tower_out = nullptr;
     int tower_path = -1;            // path of the last forward: 0 per layer, 1 cooperative launch, 2 board-resident
-    // the fused tower (64 filters): per-layer descriptors and tile flags on the device
+    // the fused tower (64 filters, only when asked for): per-layer descriptors and tile flags on the device
     void* fused_layers = nullptr; int *fused_flags = nullptr, *fused_done = nullptr; int fused_pitch = 0, fused_epoch = 0, fused_final = 0;
     bool fused = false;                         // OB200_TOWER_FUSED=2
     // the board-resident tower (64 filters, boards up to 15x15): layer descriptors, whole-board boxes
@@ -378,10 +378,10 @@ int ob200_net_finalize(ob200_net* n) {
         if (n->board8)
             if (int rc = make_board_row_maps(p8, c.board_size, c.max_batch, F, &n->act_rows[i])) return rc;
     }
-    if (!n->wide && tower_fused_smem_bytes(c.board_size, 1 + 2 * c.blocks) != 0) {
+    const char* fused_env = std::getenv("OB200_TOWER_FUSED");
+    if (fused_env && fused_env[0] == '2' && !n->wide && tower_fused_smem_bytes(c.board_size, 1 + 2 * c.blocks) != 0) {
         // one cooperative launch for the whole tower: layer descriptors with the buffer rotation of
         // forward_device baked in, and one "tile stored" flag per layer and tile
-        const char* env = std::getenv("OB200_TOWER_FUSED");
         const int L = 1 + 2 * c.blocks;
         std::vector<unsigned char> host(tower_fused_layer_bytes() * L);
         int x = 0, y = 1, z = 2;
@@ -400,7 +400,7 @@ int ob200_net_finalize(ob200_net* n) {
         n->fused_pitch = (int)(board_geom(c.board_size, c.max_batch).Ppad / 128);
         if (int rc = dev_alloc(n, &n->fused_flags, (size_t)L * n->fused_pitch, true)) return rc;
         if (int rc = dev_alloc(n, &n->fused_done, (size_t)L, true)) return rc;
-        n->fused = env && env[0] == '2';
+        n->fused = true;
     }
     if (!n->wide && n->cin_pad == 64 && tower_resident_covers(c.board_size, 1 + 2 * c.blocks)) {
         // boards stay in shared memory through all the layers: one ordinary launch
@@ -414,7 +414,7 @@ int ob200_net_finalize(ob200_net* n) {
         if (int rc = make_board_plane_maps(n->act[0], c.board_size, c.max_batch, &n->out_planes)) return rc;
         // on unless switched off; an explicit choice about the single-launch tower (OB200_TOWER_FUSED, used by
         // tests and comparisons to pick one of the other two paths) also switches it off unless it is asked for
-        n->resident = env ? env[0] != '0' : std::getenv("OB200_TOWER_FUSED") == nullptr;
+        n->resident = env ? env[0] != '0' : fused_env == nullptr;
     }
     const size_t MB = c.max_batch;
     if (!planes_policy) {
@@ -525,9 +525,11 @@ int tower_device(ob200_net* n, const void* input_bt, int B, int* out_buf, cudaSt
     if (!done && !own_input)
         if (int rc = input_map(n, input_bt, B, n->box_in, &conv_map)) return rc;
     const BoardTensorMap& in_map = own_input ? n->in_map_load : conv_map;
-    // The one-launch tower runs only when asked for (OB200_TOWER_FUSED=2): handing tiles over through flags in global
-    // memory (store complete -> flag -> poll, about 3 us a layer) now costs more than kernel boundaries at every size.
-    // 19x19, 21 layers, a launch per layer against one launch: 400 boards 276 / 308 us, 550 350 / 370, 780 503 / 541.
+    // The one-launch tower runs only when asked for (OB200_TOWER_FUSED=2), for comparison: handing tiles over through
+    // flags in global memory costs more than kernel boundaries at every size.  An evaluation with a launch per layer / one
+    // launch / one launch whose issuing warp runs as a whole, as the other kernels' do: 19x19, 21 layers, 1 board 107 /
+    // 123 / 120 us, 300 266 / 288 / 290, 600 421 / 449 / 446, 800 570 / 593 / 595; 15x15, 29 layers, 300 boards 273 / 284 /
+    // 293, 600 416 / 436 / 445, 1,000 603 / 617 / 619.
     // The tile flags carry a per-launch epoch kept on the host: a launch replayed from a captured
     // graph would see its own earlier flags, so a capturing stream gets the per-layer kernels.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;

@@ -21,9 +21,8 @@
 //     128 threads that do the arithmetic; the producer polls the halo flags of two tiles
 //     at a time and stops polling once the previous layer's published-tile count is
 //     complete (a poll with its two fences costs about 1.6 us).
-// Measured at batch 1024 (15x15, 21 layers): 19.6 us per layer instead of 22.2 us as separate
-// launches; the MMA issue period (36 MMAs, 2,440 cycles per tile) is the same in both and is
-// what bounds the kernel.
+// It is no handle's default any more (the reasons, measured, stand where net.cu chooses the path) and is kept for
+// comparison, behind OB200_TOWER_FUSED=2.
 // The three activation buffers rotate exactly as in the per-layer path, so the
 // write-after-read hazards are covered by the same flags (a tile is overwritten
 // only by a layer whose loads already waited for every reader of that tile).

@@ -79,7 +79,7 @@ struct ResidentBias { float v[kMaxLayers * kC]; };
 struct ResidentParams {
     const uint8_t* const* layers;   // [n_layers] packed weights (ob200_pack_conv3x3_weights): 9 taps x 8 KB
     int n_layers;
-    int B, S, GP, HP;
+    int B, S, HP;
     int per_tile, tiles;      // boards per tile
     int board_rows;           // rows of a board in a plane: (S + 1) * HP
     int* error;
@@ -492,7 +492,7 @@ int launch_conv_tower_resident(const BoardPlaneMaps& in, const BoardPlaneMaps& o
     ResidentBias biases;
     std::memcpy(biases.v, bias, (size_t)n_layers * kC * sizeof(float));
     ResidentParams p{};
-    p.layers = reinterpret_cast<const uint8_t* const*>(layers_dev); p.n_layers = n_layers; p.B = B; p.S = S; p.GP = S + 1; p.HP = pairs_per_row(S);
+    p.layers = reinterpret_cast<const uint8_t* const*>(layers_dev); p.n_layers = n_layers; p.B = B; p.S = S; p.HP = pairs_per_row(S);
     p.board_rows = (S + 1) * p.HP;
     // small boards share a tile once there are more of them than SMs (the last board of a tile needs no pad row below it)
     p.per_tile = std::min((kTileM + p.HP) / p.board_rows, (B + sms - 1) / sms);

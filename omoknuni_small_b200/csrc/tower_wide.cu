@@ -194,9 +194,9 @@ conv_wide_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_consta
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        // One thread issues; the loop over taps, tiles and 16-channel steps is unrolled with
-        // compile-time offsets and ring positions are kept as counters, because every integer
-        // instruction between two MMAs of this thread is time the tensor core waits.
+        // The warp runs the loop as a whole and one lane issues; taps, tiles and 16-channel steps are
+        // unrolled with compile-time offsets and ring positions are kept as counters, because every
+        // integer instruction between two MMAs is time the tensor core waits.
         {
             const uint32_t lead = elect_one();
             int tap_off[TAPS];

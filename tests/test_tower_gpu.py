@@ -433,15 +433,16 @@ def test_single_launch_tower_repeats_bit_identically(api, monkeypatch, which, B,
 
 
 def test_resident_tower_hands_over_when_the_shape_does_not_fit(api, monkeypatch):
-    """14 blocks = 29 layers of biases do not fit beside the boards in shared memory, a 19x19 board does
-    not fit at all, 128 filters are another kernel: the handle then takes one of the other paths."""
+    """The biases of 14 blocks = 29 layers do not fit the kernel's parameter, a 19x19 board does not fit
+    a tile, 128 filters are another kernel: the handle then takes a launch per layer, in batches for
+    which it once took the one-launch tower as well."""
     pick_tower(monkeypatch, "resident")
-    for S, blocks, F in ((15, 14, 64), (19, 1, 64), (15, 1, 128)):
+    for S, blocks, F, B in ((15, 14, 64, 3), (19, 1, 64, 3), (15, 1, 128, 3), (15, 14, 64, 700), (19, 1, 64, 600)):
         shapes = synth.net_tensor_shapes(S, 17, F, blocks, S * S, 2, 1)
         w = synth.make_weights(shapes, seed=3, init="torch_default", bn="random")
-        net = make_net(api, w, dict(cin=17, S=S, blocks=blocks, F=F, A=S * S, pc=2, vc=1), 4)
-        net.infer_planes(synth.make_stone_planes(3, S, 17, seed=1), api.OUT_LOGITS)
-        assert net.tower_path() in (0, 1)
+        net = make_net(api, w, dict(cin=17, S=S, blocks=blocks, F=F, A=S * S, pc=2, vc=1), B + 1)
+        net.infer_planes(synth.make_stone_planes(B, S, 17, seed=1), api.OUT_LOGITS)
+        assert net.tower_path() == 0
         net.close()
     shapes = synth.net_tensor_shapes(15, 17, 64, 13, 225, 2, 1)
     net = make_net(api, synth.make_weights(shapes, seed=3, init="torch_default", bn="random"),
