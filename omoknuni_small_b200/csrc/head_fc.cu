@@ -24,7 +24,7 @@
 // -> 221 us (that kernel took 236 us for either: eight CTAs' worth of a serial loop over 7,200 terms).
 #include "internal.h"
 #include "sm100_ptx.cuh"
-#include "head_conv.cuh"
+#include <cfloat>
 
 namespace ob200 {
 namespace {
@@ -220,7 +220,7 @@ head_fc_kernel(const SplitParams p) {
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float v = join_terms(__uint_as_float(r[j]), __uint_as_float(small[j]));
+                    const float v = __fadd_rn(__uint_as_float(r[j]), fminf(__uint_as_float(small[j]), FLT_MAX));   // (NaN -> FLT_MAX)
                     group[h * 8 + j] = __fadd_rn(group[h * 8 + j], v);
                 }
             }
@@ -237,9 +237,9 @@ head_fc_kernel(const SplitParams p) {
             const bool good = mbar_wait(empty(s), ((uint32_t)(i / kStages) & 1u) ^ 1u, abort_flag);
             if (!__all_sync(0xffffffffu, good)) { ok = false; return; }
             uint8_t* dst = smem + s * kStageBytes;
-            // terms beyond K have weights of zero, but an infinity repeated there would make NaN of them
+            // the layer's last block: terms beyond K have weights of zero, but an infinity repeated there would make NaN
             const int left = L.K - ((kb0 + i) * kStageK + kv);
-            if (left < 4) {
+            if (kb0 + i == L.k_blocks - 1 && left < 4) {
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     if (left < 1) x[r].x = 0.0f;
