@@ -139,41 +139,59 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float* red) 
     return v;
 }
 
-// Element j of row b of a layer's result: its slices of partial sums added in the layer's fixed order, fifteen loads
-// (five groups of three, or fifteen groups) in flight at a time.
-constexpr int kSliceBatch = 15;
-static_assert(kSliceBatch % kHeadFcGroup == 0, "a batch of slices is a whole number of groups");
-template <int GROUP>
-__device__ __forceinline__ float sum_slices_in(const HeadFcLayer& l, const float* p, size_t step) {
-    float total = 0.0f;
+constexpr int kTailThreads = 256;
+
+// Elements j, j + kTailThreads, ... of row b of a layer's result (the first n of N exist): its slices of partial sums
+// added in the layer's fixed order.  One element: fifteen loads (five groups of three, or fifteen groups) in flight at a
+// time; four: six each.
+template <int GROUP, int N>
+__device__ __forceinline__ void sum_slices_in(const HeadFcLayer& l, const float* p, size_t step, int n, float (&total)[N]) {
+    constexpr int kSliceBatch = N == 1 ? 15 : 6;
+    static_assert(kSliceBatch % kHeadFcGroup == 0, "a batch of slices is a whole number of groups");
     for (int s = 0; s < l.slices; s += kSliceBatch) {
-        float v[kSliceBatch];
+        float v[N][kSliceBatch];
 #pragma unroll
-        for (int k = 0; k < kSliceBatch; ++k) v[k] = s + k < l.slices ? __ldcg(p + (size_t)(s + k) * step) : 0.0f;
+        for (int e = 0; e < N; ++e)
+#pragma unroll
+            for (int k = 0; k < kSliceBatch; ++k)
+                v[e][k] = s + k < l.slices && e < n ? __ldcg(p + (size_t)(s + k) * step + e * kTailThreads) : 0.0f;
 #pragma unroll
         for (int g = 0; g < kSliceBatch; g += GROUP) {
             if (s + g >= l.slices) break;
-            float group = v[g];
 #pragma unroll
-            for (int k = g + 1; k < g + GROUP; ++k)
-                if (s + k < l.slices) group = __fadd_rn(group, v[k]);
-            total = s + g ? __fadd_rn(total, group) : group;
+            for (int e = 0; e < N; ++e) {
+                float group = v[e][g];
+#pragma unroll
+                for (int k = g + 1; k < g + GROUP; ++k)
+                    if (s + k < l.slices) group = __fadd_rn(group, v[e][k]);
+                total[e] = s + g ? __fadd_rn(total[e], group) : group;
+            }
         }
     }
-    return total;
 }
-__device__ __forceinline__ float sum_slices(const HeadFcLayer& l, int b, int B, int j) {
+template <int N>
+__device__ __forceinline__ void sum_slices(const HeadFcLayer& l, int b, int B, int j, int n, float (&total)[N]) {
     const float* p = l.part + (size_t)b * l.part_pitch + j;
     const size_t step = (size_t)B * l.part_pitch;
-    if (l.slices == 1) return __ldcg(p);
-    return l.slice_group == 1 ? sum_slices_in<1>(l, p, step) : sum_slices_in<kHeadFcGroup>(l, p, step);
+    if (l.slices == 1) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) total[e] = e < n ? __ldcg(p + e * kTailThreads) : 0.0f;
+    } else if (l.slice_group == 1) sum_slices_in<1, N>(l, p, step, n, total);
+    else sum_slices_in<kHeadFcGroup, N>(l, p, step, n, total);
+}
+__device__ __forceinline__ float sum_slices(const HeadFcLayer& l, int b, int B, int j) {
+    float total[1];
+    sum_slices(l, b, B, j, 1, total);
+    return total[0];
 }
 
 // The tails of both heads in one launch, started as a programmatic dependent of the FC kernel: CTAs [0, policy_rows)
 // finish one row of logits each (sum of the slices, bias, softmax: maximum, sum of exponentials, division), the rest
-// one board's value each.  A thread per output: what a small batch waits for is the trip to L2 for the slices.
-constexpr int kTailThreads = 256;
+// one board's value each.  A thread per output: what a small batch waits for is the trip to L2 for the slices, so a
+// thread of a longer row sums four outputs at a time (4,672 logits of one board, 450 terms: an evaluation 46.7 us with one
+// at a time, 38.6 so).
 constexpr int kTailRegs = 2;             // logits a thread keeps in registers: rows of up to 512
+constexpr int kTailAhead = 4;            // outputs a thread of a longer row sums at a time
 __global__ void __launch_bounds__(kTailThreads)
 head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __restrict__ logits, int A, int policy_rows, int softmax,
                   const HeadFcLayer val, const float* __restrict__ b1, const float* __restrict__ w2, float b2, int H, int B,
@@ -212,9 +230,18 @@ head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __
             return;
         }
         float m = -INFINITY;
-        for (int i = threadIdx.x; i < A; i += kTailThreads) {
-            if (pol.part) row[i] = __fadd_rn(sum_slices(pol, b, B, i), bp[i]);
-            m = fmaxf(m, row[i]);
+        for (int i0 = threadIdx.x; i0 < A; i0 += kTailAhead * kTailThreads) {
+            const int n = (A - i0 + kTailThreads - 1) / kTailThreads;
+            float x[kTailAhead];
+            if (pol.part) sum_slices(pol, b, B, i0, n, x);
+#pragma unroll
+            for (int k = 0; k < kTailAhead; ++k) {
+                if (k >= n) break;
+                const int i = i0 + k * kTailThreads;
+                if (pol.part) row[i] = x[k] = __fadd_rn(x[k], bp[i]);
+                else x[k] = row[i];
+                m = fmaxf(m, x[k]);
+            }
         }
         if (!softmax) return;
         m = block_reduce(m, true, red);

@@ -44,6 +44,7 @@ def head64(w, name, x):
     (15, 32, 32, 256, 225, 2),      # single chunks
     (15, 32, 32, 255, 226, 700),    # groups of chunks
     (15, 32, 32, 256, 225, 2100),   # whole layers per CTA, or groups
+    (15, 2, 1, 256, 513, 3), (15, 32, 32, 256, 1030, 2), (8, 2, 1, 64, 4672, 40), (15, 32, 32, 64, 1281, 130),   # long rows
 ])
 def test_head_fc_against_fp64(api, S, pc, vc, H, A, B):
     shapes = synth.net_tensor_shapes(S, 17, 64, 1, A, pc, vc, value_hidden=H)
