@@ -388,14 +388,25 @@ int launch_value_head_static(const void* tower, const HeadConvWeights& value_con
                          B, need, vc, S, S, H, kStaticScratchFloats);
     float* scratch = nullptr;
     if (int rc = value_head_scratch_ptr(&scratch)) return rc;
-    float* hv = scratch;                                  // [B][vc * S * S]
-    float* hidden = scratch + (size_t)B * vc * S * S;     // [B][H]
-    // every element read below is written first by the launch before it: nothing needs clearing
-    if (int rc = launch_head_conv(tower, value_conv, nullptr, hv, 0, vc * S * S, B, S, st, 64, dtype)) return rc;
-    // the layer with all its chunks in one CTA per tile: one slice, which fits the scratch
+    // Rows of a multiple of four floats, which the FC kernel reads and writes 16 bytes at a time, and the layer's chunks
+    // spread over CTAs as a forward spreads them, where the scratch holds that; rows as they are and all chunks in one CTA
+    // per tile otherwise.  Either way every element read below is written first by the launch before it, or cleared (inputs
+    // beyond K): nothing needs clearing here.  (15x15, one value channel: 149 boards 33 us with rows as they
+    // are and all chunks in one CTA, 19 so; 300 boards 29 / 19; 30x30, 64 boards 47 / 17.)
     HeadFcLayer l = value_layer;
-    l.in = hv; l.in_pitch = vc * S * S; l.part = hidden; l.part_pitch = H;
-    l.chunks_per_slice = l.chunks; l.slices = 1; l.slice_group = 1;
+    int dev = 0, sms = 0;
+    OB200_CUDA_OK(cudaGetDevice(&dev));
+    OB200_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int K = vc * S * S;
+    l.in_pitch = (K + 3) / 4 * 4; l.part_pitch = (H + 3) / 4 * 4;
+    head_fc_plan(&l, 1, B, sms);
+    auto fits = [&]() { return (size_t)B * ((size_t)l.in_pitch + (size_t)l.slices * l.part_pitch) <= kStaticScratchFloats; };
+    if (!fits() && l.chunks_per_slice == 1) { l.chunks_per_slice = kHeadFcGroup; l.slices = (l.chunks + kHeadFcGroup - 1) / kHeadFcGroup; l.slice_group = 1; }
+    if (!fits()) { l.chunks_per_slice = l.chunks; l.slices = 1; l.slice_group = 1; }
+    if (!fits()) { l.in_pitch = K; l.part_pitch = H; }
+    float* hv = scratch;                                  // [B][in_pitch]
+    l.in = hv; l.part = scratch + (size_t)B * l.in_pitch; // [slice][B][part_pitch]
+    if (int rc = launch_head_conv(tower, value_conv, nullptr, hv, 0, l.in_pitch, B, S, st, 64, dtype)) return rc;
     if (int rc = launch_head_fc(&l, 1, B, st)) return rc;
     return launch_head_tails(HeadFcLayer{}, nullptr, nullptr, 0, 0, l, b1, H, w2, b2, value_out, B, st);
 }

@@ -63,3 +63,25 @@ def test_value_head_noalloc_rejects_oversize(lib):
     net.value_head_noalloc(net.tower_output_ptr(), too_many - 1, out)   # the largest batch that fits
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy()[: too_many - 1], value.cpu().numpy()[: too_many - 1])
+
+
+@pytest.mark.parametrize("S,vc,H,B", [
+    (15, 1, 256, 149), (30, 1, 256, 64),      # rows padded to whole vectors, a chunk of the inner dimension a CTA
+    (30, 1, 256, 300),                        # groups of chunks: single ones would not fit the array
+    (19, 1, 256, 600), (15, 2, 256, 600),     # all chunks in one CTA
+    (15, 1, 255, 1092),                       # rows as they are: padded ones would not fit
+    (2, 1, 1, 3), (15, 3, 130, 7),
+])
+def test_value_head_noalloc_layouts(lib, S, vc, H, B):
+    """Each way the call lays its intermediates out in the built-in array: values equal the forward's."""
+    import torch
+    from omoknuni_small_b200 import capi
+    w = synth.make_weights(synth.net_tensor_shapes(S, 17, 64, 1, S * S, 2, vc, value_hidden=H), seed=S + B, init="torch_default", bn="random")
+    net = capi.Net(17, S, 1, 64, S * S, 2, vc, H, B).load(w)
+    bt = capi.planes_to_board_tensor(torch.from_numpy(synth.make_stone_planes(B, S, 17, seed=B, max_stones=S * S)).cuda(), 64)
+    policy, value, got = torch.empty((B, S * S), device="cuda"), torch.empty(B, device="cuda"), torch.full((B,), 7.0, device="cuda")
+    net.forward_device(bt, B, policy, value)
+    net.value_head_noalloc(net.tower_output_ptr(), B, got)
+    torch.cuda.synchronize()
+    assert torch.equal(got, value) and capi.device_error_code() == 0
+    net.close()
