@@ -22,7 +22,10 @@ using namespace ptx;
 // dropped): rows of 128 bytes per 64-channel slice into swizzled shared memory, two MMAs per 16 channels and slice
 // (see head_conv.cuh; the same products in the same order as the board-resident tower's last layer), accumulators to
 // the flattened head activations.  blockIdx.y: the group of up to 64 head channels.  HBM-bound for large batches (it
-// reads the tower's output once per group); several CTAs an SM cover one another's latency.
+// reads the tower's output once per group): the next tile's rows are on their way into registers while a tile's MMAs
+// and results are waited for, and several CTAs share an SM.  (2,048 boards of 19x19 x 128
+// channels, 2 / 1 head channels: 54.8 us with the loads behind the MMAs, 40.6 now, 32 the bytes alone; 4,096 chess
+// boards of 256 channels 58.1 -> 33.4; 512 boards of 19x19 x 128, 32 / 32 head channels, 45.1 -> 35.7.)
 constexpr int kConvThreads = 256;
 constexpr int kConvTile = 128;
 constexpr int kConvTmemCols = 128;
@@ -31,12 +34,16 @@ struct HeadConvParams {
     HeadConvWeights head;
     float *hp, *hv;
     int hp_pitch, hv_pitch;
-    int B, S, slices, tiles;
+    int B, S, tiles;
     int* error;
 };
-template <bool F16>
-__global__ void __launch_bounds__(kConvThreads)
+// CTAs an SM: 128 TMEM columns and 16 registers a slice and thread for the rows under way each.
+__host__ __device__ constexpr int conv_ctas_per_sm(int slices) { return slices == 1 ? 4 : slices == 2 ? 3 : 2; }
+// SLICES: 64-channel slices of the tower.
+template <bool F16, int SLICES>
+__global__ void __launch_bounds__(kConvThreads, conv_ctas_per_sm(SLICES))
 head_conv_kernel(const HeadConvParams p) {
+    constexpr int kRowBytes = SLICES * 128, kVecs = SLICES * kConvTile * 8 / kConvThreads;     // 16-byte pieces a thread
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
@@ -45,8 +52,8 @@ head_conv_kernel(const HeadConvParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h0 = (int)blockIdx.y * 64, hc = min(64, p.head.hc - h0), rows = (hc + 15) / 16 * 16;
     uint8_t* a_s = smem;                                                // [slice][128 rows][128 bytes]
-    uint8_t* w_s = smem + p.slices * kConvTile * 128;                   // [slice][split term][rows][128 bytes]
-    const uint32_t w_bytes = (uint32_t)(p.slices * 3 * rows * 128);
+    uint8_t* w_s = smem + SLICES * kConvTile * 128;                     // [slice][split term][rows][128 bytes]
+    const uint32_t w_bytes = (uint32_t)(SLICES * 3 * rows * 128);
     const uint32_t w_full = smem_u32(&bars[0]), done = smem_u32(&bars[1]);
     volatile int* abort_flag = &abort_s;
     if (threadIdx.x == 0) {
@@ -54,7 +61,7 @@ head_conv_kernel(const HeadConvParams p) {
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_arrive_expect_tx(w_full, w_bytes);
-        bulk_g2s(smem_u32(w_s), p.head.w + (size_t)blockIdx.y * p.slices * 3 * 64 * 128, w_bytes, w_full);
+        bulk_g2s(smem_u32(w_s), p.head.w + (size_t)blockIdx.y * SLICES * 3 * 64 * 128, w_bytes, w_full);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -67,18 +74,23 @@ head_conv_kernel(const HeadConvParams p) {
     const uint32_t tmem_base = tmem_slot;
     OB200_PDL_ENTER();
     const int GP = p.S + 1, slots = GP * GP, S2 = p.S * p.S, total = p.B * slots;
-    const size_t row_bytes = (size_t)p.slices * 128;
     const uint32_t id2 = make_idesc(F16, kConvTile, 2 * rows), id1 = make_idesc(F16, kConvTile, rows);
     const int q = warp & 3, half = warp >> 2;
     uint32_t phase = 0;
+    uint4 v[kVecs];
+    auto fetch = [&](int tile) {          // the tensor is padded to whole tiles: every row is readable
+        const uint8_t* src = p.tower + ((size_t)OB200_GUARD + (size_t)tile * kConvTile) * kRowBytes + threadIdx.x * 16;
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) v[j] = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)j * (kConvThreads * 16)));
+    };
+    if ((int)blockIdx.x < p.tiles) fetch(blockIdx.x);
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, phase ^= 1u) {
-        // the tensor is padded to whole tiles: every row is readable
-        const uint8_t* src = p.tower + ((size_t)OB200_GUARD + (size_t)tile * kConvTile) * row_bytes;
-        for (int i = threadIdx.x; i < p.slices * kConvTile * 8; i += kConvThreads) {
-            const int c = i & 7, sl = (i >> 3) % p.slices, r = (i >> 3) / p.slices;
-            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)r * row_bytes + sl * 128 + c * 16));
-            *reinterpret_cast<uint4*>(a_s + (sl * kConvTile + r) * 128 + ((c ^ (r & 7)) << 4)) = v;
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) {
+            const int i = j * kConvThreads + threadIdx.x, c = i & 7, sl = (i >> 3) % SLICES, r = (i >> 3) / SLICES;
+            *reinterpret_cast<uint4*>(a_s + (sl * kConvTile + r) * 128 + ((c ^ (r & 7)) << 4)) = v[j];
         }
+        if (tile + (int)gridDim.x < p.tiles) fetch(tile + gridDim.x);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");    // the previous tile's accumulators have been read
         __syncthreads();
@@ -86,7 +98,8 @@ head_conv_kernel(const HeadConvParams p) {
             if (mbar_wait(w_full, 0, abort_flag)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = desc_lo(smem_u32(a_s)), w = desc_lo(smem_u32(w_s));
-                for (int sl = 0; sl < p.slices; ++sl)
+                #pragma unroll
+                for (int sl = 0; sl < SLICES; ++sl)
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         const uint32_t at = a + (uint32_t)(sl * kConvTile * 8 + ks * 2), wt = w + (uint32_t)(sl * 3 * rows * 8 + ks * 2);
@@ -330,19 +343,25 @@ int launch_head_conv(const void* tower, const HeadConvWeights& head, float* hp, 
     if (g.P > 0x7fffffffLL - kConvTile) return set_error(OB200_ERR_TOO_LARGE, "head conv: batch too large");
     HeadConvParams p;
     p.tower = static_cast<const uint8_t*>(tower); p.head = head; p.hp = hp; p.hv = hv; p.hp_pitch = hp_pitch; p.hv_pitch = hv_pitch;
-    p.B = B; p.S = S; p.slices = C / 64; p.tiles = (int)(g.Ppad / kConvTile);
+    p.B = B; p.S = S; p.tiles = (int)(g.Ppad / kConvTile);
     p.error = device_error_word();
     if (!p.error) return set_error(OB200_ERR_CUDA, "head conv: cannot resolve the device error word");
     const int groups = (head.hc + 63) / 64, rows = (std::min(head.hc, 64) + 15) / 16 * 16;
-    const size_t smem = (size_t)p.slices * (kConvTile + 3 * rows) * 128 + 1024;
-    auto kernel = dtype == OB200_DTYPE_F16 ? head_conv_kernel<true> : head_conv_kernel<false>;
-    static bool configured[64][2] = {{false, false}};
-    if (dev < 0 || dev >= 64 || !configured[dev][dtype]) {
-        OB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (kConvTile + 3 * 64) * 128 + 1024));
-        if (dev >= 0 && dev < 64) configured[dev][dtype] = true;
+    const int slices = C / 64;
+    const size_t smem = (size_t)slices * (kConvTile + 3 * rows) * 128 + 1024;
+    using Kernel = void (*)(HeadConvParams);
+    static const Kernel kernels[2][4] = {
+        {head_conv_kernel<false, 1>, head_conv_kernel<false, 2>, head_conv_kernel<false, 3>, head_conv_kernel<false, 4>},
+        {head_conv_kernel<true, 1>, head_conv_kernel<true, 2>, head_conv_kernel<true, 3>, head_conv_kernel<true, 4>}};
+    const int f16 = dtype == OB200_DTYPE_F16;
+    const Kernel kernel = kernels[f16][slices - 1];
+    static bool configured[64][2][4] = {};
+    if (dev < 0 || dev >= 64 || !configured[dev][f16][slices - 1]) {
+        OB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, slices * (kConvTile + 3 * 64) * 128 + 1024));
+        if (dev >= 0 && dev < 64) configured[dev][f16][slices - 1] = true;
     }
-    // four CTAs an SM (128 TMEM columns each), where the shared memory of so many fits
-    const int per_sm = std::max(1, std::min(4, (int)(220 * 1024 / (smem + 1024))));
+    // as many CTAs an SM as their shared memory leaves room for
+    const int per_sm = std::max(1, std::min(conv_ctas_per_sm(slices), (int)(220 * 1024 / (smem + 1024))));
     OB200_CUDA_OK(launch_dependent(kernel, dim3(std::min(p.tiles, sms * per_sm), groups), dim3(kConvThreads), smem, st, p));
     counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;

@@ -66,3 +66,28 @@ def test_head_fc_against_fp64(api, S, pc, vc, H, A, B):
         part = net.infer_planes(synth.make_stone_planes(B, S, 17, seed=B, max_stones=S * S)[1:2], api.OUT_LOGITS)
         assert np.array_equal(part[0][0], logits[1]) and part[1][0] == v[1]
     net.close()
+
+
+@pytest.mark.parametrize("F,S,B,pc,vc,dtype", [
+    (64, 19, 230, 2, 1, 0),         # 719 tiles of 128 positions: CTAs of one and of two
+    (128, 19, 150, 2, 1, 1), (128, 19, 290, 33, 31, 0), (128, 15, 1, 1, 1, 0),
+    (256, 19, 100, 2, 1, 0), (256, 8, 40, 40, 30, 1),       # 70 channels: two groups
+])
+def test_head_convolution_tiles(api, F, S, B, pc, vc, dtype):
+    """The stand-alone 1x1 convolutions over towers of every width, several tiles a CTA."""
+    w = synth.make_weights(synth.net_tensor_shapes(S, 17, F, 0, 130, pc, vc, value_hidden=64), seed=F + B, init="torch_default", bn="random")
+    net = api.Net(17, S, 0, F, 130, pc, vc, 64, B, tower_dtype=dtype).load(w)
+    logits, v = net.infer_planes(synth.make_stone_planes(B, S, 17, seed=B, max_stones=S * S), api.OUT_LOGITS)
+    nb = int(api.lib().ob200_board_tensor_bytes(S, B, F))
+    raw = np.empty(nb, np.uint8)
+    api.check(api.lib().ob200_copy_to_host(raw.ctypes.data_as(ctypes.c_void_p), ctypes.c_void_p(net.tower_output_ptr()), nb))
+    x = api.board_tensor_to_planes(raw.view(np.uint16), S, B, F, dtype)[0].astype(np.float64)
+    hp, hv = head64(w, "policy", x), head64(w, "value", x)
+    wp, w1, w2 = (w[k].astype(np.float64) for k in ("policy_fc.weight", "value_fc1.weight", "value_fc2.weight"))
+    bound = BOUND + F * 2.0 ** -24
+    assert (np.abs(logits - hp @ wp.T - w["policy_fc.bias"]) <= bound * (hp @ np.abs(wp).T + np.abs(w["policy_fc.bias"]))).all()
+    hidden = np.maximum(hv @ w1.T + w["value_fc1.bias"], 0)
+    scale = (hv @ np.abs(w1).T + np.abs(w["value_fc1.bias"])) @ np.abs(w2[0]) + np.abs(w["value_fc2.bias"])
+    assert (np.abs(v - np.tanh(hidden @ w2[0] + w["value_fc2.bias"])) <= (bound + 64 * 2.0 ** -24) * scale + 2.0 ** -21).all()
+    assert api.device_error_code() == 0
+    net.close()
