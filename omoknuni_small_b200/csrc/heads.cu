@@ -198,23 +198,25 @@ __device__ __forceinline__ float sum_slices(const HeadFcLayer& l, int b, int B, 
     return total[0];
 }
 
-// The tails of both heads in one launch, started as a programmatic dependent of the FC kernel: CTAs [0, policy_rows)
-// finish one row of logits each (sum of the slices, bias, softmax: maximum, sum of exponentials, division), the rest
-// one board's value each.  A thread per output: what a small batch waits for is the trip to L2 for the slices, so a
-// thread of a longer row sums four outputs at a time (4,672 logits of one board, 450 terms: an evaluation 46.7 us with one
-// at a time, 38.6 so).
+// The tails of both heads in one launch, started as a programmatic dependent of the FC kernel: CTAs [0, policy_ctas)
+// finish a row of logits each (sum of the slices, bias, softmax: maximum, sum of exponentials, division), or a share of a
+// long one that is not normalised, the rest one board's value each.  A thread per output: what a small batch waits for is
+// the trip to L2 for the slices, so a thread of a longer row sums four outputs at a time and long rows of plain logits are
+// shared out.  4,672 logits of one board, an evaluation: 450 terms 46.7 us with one output at a time, 38.6 with four, 32.9
+// shared out as well; 128 terms 33.0, 30.6, 26.7.
 constexpr int kTailRegs = 2;             // logits a thread keeps in registers: rows of up to 512
 constexpr int kTailAhead = 4;            // outputs a thread of a longer row sums at a time
+constexpr int kTailSpan = kTailAhead * kTailThreads;     // a CTA's share of a longer row that is not normalised
 __global__ void __launch_bounds__(kTailThreads)
-head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __restrict__ logits, int A, int policy_rows, int softmax,
+head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __restrict__ logits, int A, int policy_ctas, int row_parts, int softmax,
                   const HeadFcLayer val, const float* __restrict__ b1, const float* __restrict__ w2, float b2, int H, int B,
                   float* __restrict__ value, const int* error_word, int* error_out) {
     __shared__ float red[kTailThreads / 32];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (error_out && blockIdx.x == 0 && threadIdx.x == 0) *error_out = __ldcg(error_word);
-    if ((int)blockIdx.x < policy_rows) {
-        const int b = blockIdx.x;
+    if ((int)blockIdx.x < policy_ctas) {
+        const int b = (int)blockIdx.x / row_parts;
         float* row = logits + (size_t)b * A;
         if (A <= kTailRegs * kTailThreads) {
             float x[kTailRegs];
@@ -243,7 +245,8 @@ head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __
             return;
         }
         float m = -INFINITY;
-        for (int i0 = threadIdx.x; i0 < A; i0 += kTailAhead * kTailThreads) {
+        const int from = ((int)blockIdx.x - b * row_parts) * kTailSpan, to = row_parts > 1 ? min(A, from + kTailSpan) : A;
+        for (int i0 = from + threadIdx.x; i0 < to; i0 += kTailSpan) {
             const int n = (A - i0 + kTailThreads - 1) / kTailThreads;
             float x[kTailAhead];
             if (pol.part) sum_slices(pol, b, B, i0, n, x);
@@ -264,7 +267,7 @@ head_tails_kernel(const HeadFcLayer pol, const float* __restrict__ bp, float* __
         const float inv = 1.0f / s;
         for (int i = threadIdx.x; i < A; i += kTailThreads) row[i] = expf(row[i] - m) * inv;
     } else {
-        const int b = (int)blockIdx.x - policy_rows;
+        const int b = (int)blockIdx.x - policy_ctas;
         float s = 0.0f;
         for (int i = threadIdx.x; i < H; i += kTailThreads) s = fmaf(relu_keep_nan(__fadd_rn(sum_slices(val, b, B, i), b1[i])), w2[i], s);
         s = block_reduce(s, false, red);
@@ -278,8 +281,9 @@ int launch_head_tails(const HeadFcLayer& policy, const float* bp, float* policy_
                       const HeadFcLayer& value, const float* b1, int H, const float* w2, float b2, float* value_out, int B,
                       cudaStream_t st, int* error_out) {
     const int rows = policy_out && (policy.part || softmax) ? B : 0;
-    OB200_CUDA_OK(launch_dependent(head_tails_kernel, dim3((unsigned)(rows + B)), dim3(kTailThreads), 0, st, policy, bp,
-                                   policy_out, policy_size, rows, softmax, value, b1, w2, b2, H, B, value_out,
+    const int parts = softmax || policy_size <= kTailRegs * kTailThreads ? 1 : (policy_size + kTailSpan - 1) / kTailSpan;
+    OB200_CUDA_OK(launch_dependent(head_tails_kernel, dim3((unsigned)(rows * parts + B)), dim3(kTailThreads), 0, st, policy, bp,
+                                   policy_out, policy_size, rows * parts, parts, softmax, value, b1, w2, b2, H, B, value_out,
                                    (const int*)(error_out ? device_error_word() : nullptr), error_out));
     counters().launches.fetch_add(1, std::memory_order_relaxed);
     return OB200_OK;

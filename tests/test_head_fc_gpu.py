@@ -61,6 +61,11 @@ def test_head_fc_against_fp64(api, S, pc, vc, H, A, B):
     scale = (hv @ np.abs(w1).T + np.abs(w["value_fc1.bias"])) @ np.abs(w2[0]) + np.abs(w["value_fc2.bias"])
     # tanh is a contraction; its own fp32 error and the H additions of the last layer come on top
     assert (np.abs(v - np.tanh(hidden @ w2[0] + w["value_fc2.bias"])) <= (BOUND + H * 2.0 ** -24) * scale + 2.0 ** -21).all()
+    # probabilities of the same logits; fp32: exponentials within 2 ulp of arguments rounded to 2^-24 of their size, A additions
+    probs, _ = net.infer_planes(synth.make_stone_planes(B, S, 17, seed=B, max_stones=S * S))
+    e = np.exp(logits.astype(np.float64) - logits.max(1, keepdims=True))
+    spread = np.abs(logits - logits.max(1, keepdims=True)).max()
+    assert (np.abs(probs - e / e.sum(1, keepdims=True)) <= e / e.sum(1, keepdims=True) * (A + 16 + 2 * spread) * 2.0 ** -23).all()
     # a position's result does not depend on the batch it comes in
     if B > 2:
         part = net.infer_planes(synth.make_stone_planes(B, S, 17, seed=B, max_stones=S * S)[1:2], api.OUT_LOGITS)
