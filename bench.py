@@ -196,20 +196,31 @@ def time_wide_net(capi, torch, wc, dev, local, rank, flush, timed, steps):
     for _ in range(3):
         fwd()
     ms = float(np.mean(timed(fwd, steps)))
-    rngw = np.random.default_rng(0)
-    wp = torch.from_numpy(capi.pack_conv3x3(rngw.normal(0, 0.03, (F, F, 3, 3)).astype(np.float32), None, F).view(np.int16)).to(dev)
-    bias = torch.zeros(F, device=dev)
-    n_el = int(capi.lib().ob200_board_tensor_bytes(S, B, F)) // 2
-    bufs = [torch.zeros(n_el, dtype=torch.int16, device=dev) for _ in range(3)]
-    reps = 10
+    if S == 8:
+        # 8x8 boards have a kernel of their own, which the one-layer entry point does not take: the tower as it runs, a
+        # launch per layer (stem and 2 * blocks convolutions)
+        convs = 1 + 2 * wc["blocks"]
+        conv_flops = 2.0 * S * S * 9 * F * (wc["cin"] + (convs - 1) * F) * B / convs
 
-    def conv_loop():
-        for i in range(reps):
-            capi.conv3x3(bufs[i % 3], wp, bias, bufs[(i + 2) % 3], B, S, F, F, True, out=bufs[(i + 1) % 3])
+        def conv_loop():
+            net.tower_device(bt, B)
+        reps = convs
+    else:
+        rngw = np.random.default_rng(0)
+        wp = torch.from_numpy(capi.pack_conv3x3(rngw.normal(0, 0.03, (F, F, 3, 3)).astype(np.float32), None, F).view(np.int16)).to(dev)
+        bias = torch.zeros(F, device=dev)
+        n_el = int(capi.lib().ob200_board_tensor_bytes(S, B, F)) // 2
+        bufs = [torch.zeros(n_el, dtype=torch.int16, device=dev) for _ in range(3)]
+        reps = 10
+        conv_flops = 2.0 * S * S * 9 * F * F * B
+
+        def conv_loop():
+            for i in range(reps):
+                capi.conv3x3(bufs[i % 3], wp, bias, bufs[(i + 2) % 3], B, S, F, F, True, out=bufs[(i + 1) % 3])
     conv_loop()
     conv_ms = float(np.mean(timed(conv_loop, 3))) / reps
     net.close()
-    return dict(cfg=wc, ms=ms, conv_ms=conv_ms)
+    return dict(cfg=wc, ms=ms, conv_ms=conv_ms, conv_flops=conv_flops)
 
 
 def wide_report(wr, world, peaks):
@@ -220,17 +231,18 @@ def wide_report(wr, world, peaks):
                  + 2 * S2 * wc["F"] * wc["pc"])
     else:
         flops = synth.net_flops_per_eval(wc["S"], wc["cin"], wc["F"], wc["blocks"], wc["A"], wc["pc"], wc["vc"])
-    conv_tf = 2.0 * S2 * 9 * wc["F"] * wc["F"] * wc["B"] / (wr["conv_ms"] * 1e-3) / 1e12
+    conv_tf = wr["conv_flops"] / (wr["conv_ms"] * 1e-3) / 1e12
     evals = world * wc["B"] / (wr["ms"] * 1e-3)
     return {"workload": wc["name"], "batch_per_gpu": wc["B"], "value": evals, "unit": UNIT, "ms_per_step": wr["ms"],
             "tower_tflops": evals / world * flops / 1e12, "flops_per_eval": flops,
             "weights": "libtorch-default init seed 42, random BatchNorm", "input": "device-resident board tensor",
-            "roofline": {"kernel": f"conv_wide_kernel ({wc['F']}->{wc['F']}, residual+ReLU)", "bound": "tensor",
+            "roofline": {"kernel": (f"conv_board8_kernel ({wc['F']} channels, mean of the tower's {1 + 2 * wc['blocks']} launches)" if wc["S"] == 8
+                                    else f"conv_wide_kernel ({wc['F']}->{wc['F']}, residual+ReLU)"), "bound": "tensor",
                          "achieved": conv_tf, "peak": peaks["bf16_burst"], "unit": "TFLOP/s",
                          "frac": conv_tf / peaks["bf16_burst"],
                          "frac_of_sustained": conv_tf / peaks["bf16_sustained"] if peaks["bf16_sustained"] else None,
                          "us_per_launch": wr["conv_ms"] * 1e3,
-                         "flops": "real board cells only; the padded (S+1)^2 grid the kernel computes is not counted"}}
+                         "flops": "real board cells only; what a kernel computes on padding is not counted"}}
 
 
 def wide_only(args):
@@ -389,7 +401,7 @@ def gpu_arm(args):
         tower_loop_o()
         tower_o_ms = float(np.mean(timed(tower_loop_o, 5))) / tower_reps
         net_o.close()
-        # ---- the same network at the other batch sizes of the configurations (256: configs[0]; 4096) ----
+        # ---- the same network at the other batch sizes of the configurations (256 and 4096) ----
         sweep = []
         if not args.no_sweep:
             net_sw = capi.Net(17, 15, NET["blocks"], 64, 225, NET["policy_head_ch"], NET["value_head_ch"], 256, 4096, local,
@@ -558,13 +570,13 @@ def gpu_arm(args):
                          "frac_of_sustained": tower_tf / peaks["bf16_sustained"] if peaks["bf16_sustained"] else None,
                          "peak_source": peaks["source"] + " (burst: kernel timed alone)", "us_per_launch": tower_ms * 1e3,
                          "launches_per_tower": int(tower_launches), "flops_per_launch": tower_flops,
-                         # DRAM bytes per launch from the ncu captures at batch 512, scaled by the boards processed: the
+                         # DRAM bytes per launch from ncu captures at batch 512, scaled by the boards processed: the
                          # input tensor and the weights are read; the board-resident tower writes nothing back to DRAM
                          # (its output stays in L2), the cooperative-launch tower works out of L2 after the first layer
                          "traffic": {2: 18.38e6, 1: 21.05e6}.get(tower_path, 21 * 33.66e6) * B / 512.0, "traffic_unit": "bytes/launch",
                          # the same kernel as the network step launches it (input planes written from the move histories,
                          # no input tensor): the packed weights once and 34 bytes of history per board
-                         "traffic_in_step": 1.765e6 + 34.0 * B,
+                         "traffic_in_step": 1.608e6 + 34.0 * B,
                          "traffic_source": {2: "profiles/conv_tower_resident_kernel_gomoku15_batch512.md (scaled by batch)",
                                             1: "profiles/conv_tower_kernel_gomoku15_batch512.md (scaled by batch)"}.get(
                                                 tower_path, "profiles/conv3x3_kernel_gomoku15_batch512.md (21 launches, scaled by batch)")},
@@ -582,7 +594,7 @@ def gpu_arm(args):
                          "traffic": 33.66e6 * B / 512.0, "traffic_unit": "bytes/launch",
                          "traffic_source": "profiles/conv3x3_kernel_gomoku15_batch512.md (scaled by batch)"},
             # the stand-alone encoder launch: 8 KB of 17-plane positions per board (225 x 17 x 2 B + 34 B of history in) by the
-            # north star's count; the kernel writes the whole padded 64-channel board tensor (32 KB per board)
+            # benchmark's count; the kernel writes the whole padded 64-channel board tensor (32 KB per board)
             "encoder": {"kernel": "encode_gomoku_board_kernel", "us_per_launch": enc_ms * 1e3, "boards": B,
                         "algorithmic_gbs": B * (225 * 17 * 2 + 34) / (enc_ms * 1e-3) / 1e9,
                         "written_gbs": B * 256 * 64 * 2 / (enc_ms * 1e-3) / 1e9,
