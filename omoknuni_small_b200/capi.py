@@ -420,7 +420,7 @@ class Net:
 
     def infer_gomoku(self, history, n_hist, to_move, out_kind=OUT_PROBS, out=None):
         """out: optional (policy [B, A] float32, value [B] float32) numpy arrays to fill; arrays in
-        page-locked memory are written by the copy engine directly."""
+        page-locked memory are written by the copy engine directly (small results go through the handle's own)."""
         h = np.ascontiguousarray(history, np.int16)
         nh = np.ascontiguousarray(n_hist, np.uint8)
         tm = np.ascontiguousarray(to_move, np.uint8)
